@@ -38,8 +38,23 @@ cudaError_t Context::alloc(void** p, size_t bytes) {
   return e;
 }
 
+void Context::release(void* p) {
+  const auto it = std::find(allocations.begin(), allocations.end(), p);
+  if (it == allocations.end()) return;
+  cudaFree(p);
+  allocations.erase(it);
+}
+
 void Context::release_all() {
   invalidate_graph();
+  if (h_status != nullptr) cudaFreeHost(h_status);
+  h_status = nullptr;
+  d_list = d_list_cnt = nullptr;
+  d_vmax = nullptr;
+  lists = false;
+  list_redos = 0;
+  list_cap_scale = 1.0;
+  list_margin = 0.005f;
   for (void* p : allocations) cudaFree(p);
   allocations.clear();
   d_tanks = nullptr;
@@ -65,9 +80,9 @@ void Context::release_all() {
 }
 
 void Context::invalidate_graph() {
-  if (graph_exec != nullptr) {
-    cudaGraphExecDestroy(graph_exec);
-    graph_exec = nullptr;
+  for (cudaGraphExec_t& g : graph_exec) {
+    if (g != nullptr) cudaGraphExecDestroy(g);
+    g = nullptr;
   }
 }
 
@@ -521,12 +536,36 @@ int upload_particles(tg_context* ctx, int32_t n_tanks, const tg_tank* tanks,
     D.visc_eps2_f = static_cast<float>(D.visc_eps2);
     D.c02_f = static_cast<float>(D.cs0 * D.cs0);
     {
+      const double unit = cs / 268435456.0;  // 2^-28 cells
+      const bool wendland = C.P.kernel >= TG_KERNEL_WENDLAND_C2;
+      // f'(q)/q of the Wendland kernels without the polynomial of list_g.
+      const double lead = C.P.kernel == TG_KERNEL_WENDLAND_C2   ? -5.0
+                          : C.P.kernel == TG_KERNEL_WENDLAND_C4 ? -14.0 / 3.0
+                                                                : -2.75;
+      D.list_inv_unit = 1.0 / unit;
+      D.list_s = wendland ? T.m * D.wg * D.hinv * lead : T.m * D.wg;
+      D.list_s_f = static_cast<float>(wendland ? D.list_s * unit : D.list_s);
+      D.list_unit_f = static_cast<float>(unit);
+      D.list_hq_f = static_cast<float>(unit * D.hinv);
+      D.list_ah_f = static_cast<float>(C.P.alpha * T.h / unit);
+      D.list_eps2_f = static_cast<float>(D.visc_eps2 / (unit * unit));
+      D.list_dk_f = static_cast<float>(D.diff_k / unit);
+      D.list_mu2_f = static_cast<float>(2.0 * C.P.mu / unit);
+      D.list_lo_f = static_cast<float>(R * R * (1.0 - 1.0 / 16384.0) / (unit * unit));
+      D.list_hi_f = static_cast<float>(R * R * (1.0 + 1.0 / 16384.0) / (unit * unit));
+      D.R_f = static_cast<float>(R);
+      D.inv_rho0_f = static_cast<float>(1.0 / T.rho0);
+    }
+    {
       const double rc = R * (1.0 + 1.0 / 4096.0);
       D.cull_r2_f = static_cast<float>(rc * rc);
       double extent = 0.0;
       for (int k = 0; k < dim; ++k) extent = std::max(extent, D.nc[k] * cs);
       const double rs = rc + extent / 524288.0;
       D.wall_skip_r2_f = static_cast<float>(rs * rs);
+      // Rounding of the tank-local FP32 coordinates, of the row clips and
+      // of the squared distance: 8 ulps of the extent and R / 2048.
+      D.list_slack_f = static_cast<float>(extent / 2097152.0 + R / 2048.0);
     }
     id_base[t] = static_cast<uint32_t>(base);
     wall_from[t] = static_cast<uint32_t>(base + T.n_fluid);
@@ -559,7 +598,10 @@ int upload_particles(tg_context* ctx, int32_t n_tanks, const tg_tank* tanks,
   TG_CUDA(&C, A(C.d_dt, sizeof(double) * n_tanks));
   TG_CUDA(&C, A(C.d_dt_last, sizeof(double) * n_tanks));
   TG_CUDA(&C, A(C.d_time, sizeof(double) * n_tanks));
-  TG_CUDA(&C, A(C.d_err, sizeof(uint32_t)));
+  TG_CUDA(&C, A(C.d_err, 4 * sizeof(uint32_t)));
+  TG_CUDA(&C, A(C.d_vmax, sizeof(unsigned) * n_tanks));
+  TG_CUDA(&C, cudaMallocHost(&C.h_status, 4 * sizeof(uint32_t) + sizeof(double) * n_tanks));
+  C.steps_done = 0;
   TG_CUDA(&C, A(C.d_wall_count, 2 * sizeof(uint32_t)));
   TG_CUDA(&C, A(C.d_fbox, sizeof(unsigned) * 6 * n_tanks));
   TG_CUDA(&C, A(C.keys_a, sizeof(uint32_t) * nn));
@@ -612,7 +654,8 @@ int upload_particles(tg_context* ctx, int32_t n_tanks, const tg_tank* tanks,
                               cudaMemcpyHostToDevice, s));
   TG_CUDA(&C, cudaMemcpyAsync(C.d_time, zeros.data(), sizeof(double) * n_tanks,
                               cudaMemcpyHostToDevice, s));
-  TG_CUDA(&C, cudaMemsetAsync(C.d_err, 0, sizeof(uint32_t), s));
+  TG_CUDA(&C, cudaMemsetAsync(C.d_err, 0, 4 * sizeof(uint32_t), s));
+  TG_CUDA(&C, cudaMemsetAsync(C.d_vmax, 0, sizeof(unsigned) * n_tanks, s));
   if (n > 0) {
     TG_CUDA(&C, cudaMemcpyAsync(C.d_stage, r, sizeof(double) * n * dim,
                                 cudaMemcpyHostToDevice, s));
@@ -682,66 +725,110 @@ int tg_prepare(tg_context* ctx) {
   return TG_OK;
 }
 
+}  // extern "C"
+
+namespace {
+
+// Enqueue n steps: graph replays (captured on first use), or direct launches
+// while profiling, without graphs, or where a stopped step is repeated.
+int enqueue_steps(Context& C, int32_t n, bool direct) {
+  TG_CUDA(&C, C.engine->ensure_keys(C));
+  if (direct) {
+    for (int32_t i = 0; i < n; ++i) {
+      TG_CUDA(&C, C.engine->enqueue_step(C));
+      C.prof.stages += tg::force_passes(C.P.integrator);
+      C.prof.forces_launches += tg::force_passes(C.P.integrator);
+    }
+    return TG_OK;
+  }
+  for (int32_t i = 0; i < n; ++i) {
+    // The re-sort is taken only in the home order of an earlier sort, a
+    // host-side choice baked into the graph: one graph for each.
+    const int g = C.order_valid ? 1 : 0;
+    if (C.graph_exec[g] == nullptr) {
+      cudaGraph_t graph = nullptr;
+      const int64_t before = C.launches;
+      TG_CUDA(&C, cudaStreamBeginCapture(C.stream, cudaStreamCaptureModeThreadLocal));
+      const cudaError_t e = C.engine->enqueue_step(C);
+      const cudaError_t e2 = cudaStreamEndCapture(C.stream, &graph);
+      if (e != cudaSuccess) return cuda_fail(&C, e, "enqueue_step");
+      if (e2 != cudaSuccess) return cuda_fail(&C, e2, "cudaStreamEndCapture");
+      C.graph_kernels[g] = C.launches - before;
+      C.launches = before;
+      const cudaError_t e3 = cudaGraphInstantiate(&C.graph_exec[g], graph, 0);
+      cudaGraphDestroy(graph);
+      if (e3 != cudaSuccess) {
+        C.graph_exec[g] = nullptr;
+        return cuda_fail(&C, e3, "cudaGraphInstantiate");
+      }
+    }
+    TG_CUDA(&C, cudaGraphLaunch(C.graph_exec[g], C.stream));
+    C.launches += C.graph_kernels[g];
+    C.keys_valid = true;
+    C.order_valid = true;
+  }
+  return TG_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
 int tg_step(tg_context* ctx, int32_t n_steps, double* dt_out) {
   if (ctx == nullptr || n_steps < 0) return TG_ERR_INVALID_ARGUMENT;
   Context& C = ctx->c;
   if (!C.uploaded) return fail(&C, TG_ERR_NOT_READY, "no particles uploaded");
-  if (n_steps > 0 && C.n > 0) {
-    TG_CUDA(&C, C.engine->ensure_keys(C));
-    if (C.use_graph && !C.profile) {
-      // The re-sort is taken only in the home order of an earlier sort, a
-      // host-side choice baked into the graph: run a step directly when the
-      // order is not there yet, and capture again when it changed.
-      if (C.graph_exec != nullptr && C.graph_order != C.order_valid) C.invalidate_graph();
-      if (!C.order_valid && C.P.resort != 0 && n_steps > 1) {
-        TG_CUDA(&C, C.engine->enqueue_step(C));
-        --n_steps;
-        C.prof.steps += 1;
-      }
-      if (C.graph_exec == nullptr) {
-        C.graph_order = C.order_valid;
-        cudaGraph_t graph = nullptr;
-        const int64_t before = C.launches;
-        TG_CUDA(&C, cudaStreamBeginCapture(C.stream,
-                                           cudaStreamCaptureModeThreadLocal));
-        const cudaError_t e = C.engine->enqueue_step(C);
-        const cudaError_t e2 = cudaStreamEndCapture(C.stream, &graph);
-        if (e != cudaSuccess) return cuda_fail(&C, e, "enqueue_step");
-        if (e2 != cudaSuccess) return cuda_fail(&C, e2, "cudaStreamEndCapture");
-        C.graph_kernels = C.launches - before;
-        C.launches = before;
-        const cudaError_t e3 = cudaGraphInstantiate(&C.graph_exec, graph, 0);
-        cudaGraphDestroy(graph);
-        if (e3 != cudaSuccess) {
-          C.graph_exec = nullptr;
-          return cuda_fail(&C, e3, "cudaGraphInstantiate");
-        }
-      }
-      for (int32_t i = 0; i < n_steps; ++i) {
-        TG_CUDA(&C, cudaGraphLaunch(C.graph_exec, C.stream));
-        C.launches += C.graph_kernels;
-      }
-    } else {
-      for (int32_t i = 0; i < n_steps; ++i) {
-        TG_CUDA(&C, C.engine->enqueue_step(C));
-        C.prof.stages += tg::force_passes(C.P.integrator);
-        C.prof.forces_launches += tg::force_passes(C.P.integrator);
-      }
-    }
+  auto* status = static_cast<uint32_t*>(C.h_status);
+  auto* last_dt = reinterpret_cast<double*>(status + 4);
+  const bool steps = n_steps > 0 && C.n > 0;
+  if (steps) {
+    const bool had = C.lists;
+    TG_CUDA(&C, C.engine->prepare_lists(C));
+    if (C.lists != had) C.invalidate_graph();
     C.prof.steps += n_steps;
     // With shifting, the post-integration prepare left the walls as the
     // reference leaves them (extrapolated before the shift); otherwise the
     // reference's closing prepare runs on the next density download.
     C.walls_fresh = C.P.post_integrate == TG_POST_SHIFTING;
   }
-  TG_CUDA(&C, cudaStreamSynchronize(C.stream));
-  C.drain_profile();
-  uint32_t err = 0;
-  TG_CUDA(&C, cudaMemcpy(&err, C.d_err, sizeof(err), cudaMemcpyDeviceToHost));
-  if (dt_out != nullptr) {
-    TG_CUDA(&C, cudaMemcpy(dt_out, C.d_dt_last, sizeof(double) * C.ntanks,
-                           cudaMemcpyDeviceToHost));
+  bool direct = !C.use_graph || C.profile;
+  int32_t left = steps ? n_steps : 0;
+  for (;;) {
+    if (left > 0) {
+      const int st = enqueue_steps(C, left, direct);
+      if (st != TG_OK) return st;
+    }
+    TG_CUDA(&C, cudaMemcpyAsync(status, C.d_err, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                                C.stream));
+    TG_CUDA(&C, cudaMemcpyAsync(last_dt, C.d_dt_last, sizeof(double) * C.ntanks,
+                                cudaMemcpyDeviceToHost, C.stream));
+    TG_CUDA(&C, cudaStreamSynchronize(C.stream));
+    C.drain_profile();
+    const uint32_t done = status[2] - C.steps_done;
+    C.steps_done = status[2];
+    if (status[1] == 0u) break;
+    // A step could not be finished on its lists (pairlist.cuh): it and those
+    // behind it left the state alone.  The rest of this call sorts in every
+    // stage; later calls get longer lists or a wider margin.
+    const uint32_t why = status[1];
+    left -= static_cast<int32_t>(done);
+    TG_CUDA(&C, cudaMemsetAsync(C.d_err + 1, 0, sizeof(uint32_t), C.stream));
+    C.keys_valid = false;
+    C.order_valid = false;
+    C.lists = false;
+    C.invalidate_graph();
+    C.list_redos += 1;
+    if ((why & tg::kStopMoved) != 0u) C.list_margin *= 2.f;
+    if ((why & tg::kStopCapacity) != 0u) {
+      C.list_cap_scale *= 1.5;
+      C.release(C.d_list);
+      C.release(C.d_list_cnt);
+      C.d_list = C.d_list_cnt = nullptr;
+    }
+    direct = true;
   }
+  if (dt_out != nullptr) std::memcpy(dt_out, last_dt, sizeof(double) * C.ntanks);
+  const uint32_t err = status[0];
   if (err & (TG_DEV_NONFINITE_STATE | TG_DEV_BAD_DT)) {
     return fail(&C, TG_ERR_DEVICE_STATE,
                 "device error word " + std::to_string(err) +

@@ -15,6 +15,10 @@ namespace tg {
 
 struct Context;
 
+// Why a step could not be finished on its neighbour lists (status word [1]).
+constexpr uint32_t kStopMoved = 1u;     // a particle moved beyond the bound
+constexpr uint32_t kStopCapacity = 2u;  // a list outgrew its capacity
+
 // Force passes per step of an integrator.
 inline int force_passes(int integrator) {
   switch (integrator) {
@@ -61,6 +65,9 @@ struct EngineBase {
   virtual cudaError_t enqueue_sumdens(Context& C, int pos_precision,
                                       double* rho, int32_t* counts,
                                       uint64_t* hashes) = 0;
+  // Allocate the step's neighbour lists if it runs on them and has none yet
+  // (C.lists says whether it does).
+  virtual cudaError_t prepare_lists(Context& C) = 0;
   // Whether the force pass has a variant with `team` lanes per target.
   virtual bool supports_team(int team) const = 0;
 };
@@ -131,7 +138,12 @@ struct Context {
   double* d_dt = nullptr;
   double* d_dt_last = nullptr;
   double* d_time = nullptr;
+  // Status words: [0] TG_DEV_* bits, [1] why a step stopped (kStop*), [2]
+  // steps finished.
   uint32_t* d_err = nullptr;
+  unsigned* d_vmax = nullptr;  // per tank: max |v| of the step (float bits)
+  void* h_status = nullptr;    // page-locked: the status words, dt per tank
+  uint32_t steps_done = 0;     // status word [2] as last read
   uint32_t* d_wall_count = nullptr;  // [0] walls listed, [1] walls near fluid
   // Per tank: order-preserving encodings of the fluid bounding box of the
   // current stage (FP32, rounded outwards), mins [ntanks x 3] then maxes.
@@ -164,15 +176,26 @@ struct Context {
   const uint32_t* sorted_keys = nullptr;
   const uint32_t* perm = nullptr;
 
-  // CUDA graph of one step.
+  // CUDA graphs of one step, from a home state out of order (full sort) [0]
+  // and in the order of its last sort [1].
   bool use_graph = true;
-  cudaGraphExec_t graph_exec = nullptr;
-  int64_t graph_kernels = 0;
+  cudaGraphExec_t graph_exec[2] = {nullptr, nullptr};
+  int64_t graph_kernels[2] = {0, 0};
+
+  // Neighbour lists of the step (pairlist.cuh): whether steps run on them,
+  // their capacity per particle, the acceleration margin and how often a
+  // step had to be repeated (lists_max_redo: no lists until the next upload).
+  bool lists = false;
+  int list_cap = 0;
+  double list_cap_scale = 1.0;
+  float list_margin = 0.005f;
+  int list_redos = 0;
+  uint32_t* d_list = nullptr;
+  uint32_t* d_list_cnt = nullptr;
 
   bool walls_fresh = false;
   bool keys_valid = false;  // home keys match the home positions
   bool order_valid = false; // home state in the order of its last sort (pkey)
-  bool graph_order = false; // order_valid when the step graph was captured
 
   // Profiling.
   bool profile = false;
@@ -184,6 +207,7 @@ struct Context {
   std::string last_error;
 
   cudaError_t alloc(void** p, size_t bytes);
+  void release(void* p);  // one buffer of alloc
   void release_all();
   void invalidate_graph();
 

@@ -6,6 +6,7 @@
 
 #include "engine.cuh"
 #include "fluid.cuh"
+#include "pairlist.cuh"
 #include "post.cuh"
 #include "sort.cuh"
 
@@ -17,7 +18,8 @@ inline unsigned grid_for(int64_t n, int block) {
 
 // Compile-time physics preset of the compensated force kernel for params.
 inline int physics_preset(const tg_params& P) {
-  if (!P.kahan) return kPhysGeneric;
+  // The presets' pair sums take the Tait law with xi = 7 for granted.
+  if (!P.kahan || P.xi != 7.0 || P.eos != TG_EOS_TAIT) return kPhysGeneric;
   if (P.viscosity == TG_VISC_MONAGHAN && P.diffusion == TG_DIFF_MOLTENI) {
     return kPhysTextbook;
   }
@@ -26,6 +28,11 @@ inline int physics_preset(const tg_params& P) {
   }
   return kPhysGeneric;
 }
+
+// Longest list of a particle, and how many steps may have to be repeated
+// before a context goes without lists until the next upload.
+constexpr double kListMaxCap = 1024.0;
+constexpr int kListMaxRedos = 4;
 
 // Kernels with multi-lane force variants: the two the shipped parameter
 // sets use (Wendland C2 and C4); the others run one lane per target.
@@ -75,6 +82,8 @@ class Engine final : public EngineBase {
       }
       A(U.rho, n);
     }
+    posrec_b_ = nullptr;
+    datrec_b_ = nullptr;
     // Two spare records: the staged force pass copies row segments rounded
     // out to 16-byte boundaries, which may reach one record past the end.
     A(posrec_, n + 2);
@@ -113,8 +122,59 @@ class Engine final : public EngineBase {
     return cudaGetLastError();
   }
 
+  cudaError_t prepare_lists(Context& C) override {
+    C.lists = false;
+    const bool rk = C.P.integrator == TG_SSPRK2 || C.P.integrator == TG_SSPRK3;
+    if (!rk || C.n == 0 || C.n_fluid == 0 || C.list_redos >= kListMaxRedos) return cudaSuccess;
+    if (C.d_list == nullptr) {
+      // Entries per particle: those of a ball of the list's radius at the
+      // reference density, with room for disorder and compression; the
+      // largest over the tanks.
+      double most = 0.0;
+      for (size_t t = 0; t < C.tanks.size(); ++t) {
+        const TankDev& T = C.tankdev[t];
+        const double R = 1.06 * T.R_f;
+        const double ball = D == 2 ? 3.14159265358979 * R * R : 4.18879020478639 * R * R * R;
+        most = std::max(most, ball * T.rho0 / T.m);
+        // Tank-local FP32 coordinates must resolve the radius.
+        if (T.list_slack_f > 0.02f * T.R_f) return cudaSuccess;
+      }
+      const double cap = std::ceil((1.3 * most + 12.0) * C.list_cap_scale / 4.0) * 4.0;
+      const int64_t tiles = (C.n + 31) / 32;
+      const double bytes = 32.0 * static_cast<double>(tiles) *
+                           (4.0 * cap + sizeof(uint32_t) + sizeof(DatRec) + sizeof(PosRec));
+      size_t avail = 0, total = 0;
+      if (cudaMemGetInfo(&avail, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return cudaSuccess;
+      }
+      // Lists are an option: they leave most of the memory to others.
+      if (!(cap <= kListMaxCap) || bytes > 0.35 * static_cast<double>(avail)) return cudaSuccess;
+      C.list_cap = static_cast<int>(cap);
+      cudaError_t e = C.alloc(reinterpret_cast<void**>(&C.d_list),
+                              sizeof(uint32_t) * 32 * static_cast<size_t>(tiles) * C.list_cap);
+      if (e == cudaSuccess) {
+        e = C.alloc(reinterpret_cast<void**>(&C.d_list_cnt), sizeof(uint32_t) * C.n);
+      }
+      if (e == cudaSuccess && datrec_b_ == nullptr) {
+        e = C.alloc(reinterpret_cast<void**>(&datrec_b_), sizeof(DatRec) * C.n);
+        if (e == cudaSuccess && F == TG_FP64) {
+          e = C.alloc(reinterpret_cast<void**>(&posrec_b_), sizeof(PosRec) * C.n);
+        }
+      }
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        release_lists(C);
+        return cudaSuccess;
+      }
+    }
+    C.lists = true;
+    return cudaSuccess;
+  }
+
   cudaError_t enqueue_step(Context& C) override {
     if (C.n == 0) return cudaSuccess;
+    if (C.lists) return enqueue_list_step(C);
     static const double w3[3] = {1.0, 1.0 / 4.0, 2.0 / 3.0};
     static const double w2[2] = {1.0, 1.0 / 2.0};
     const int integ = C.P.integrator;
@@ -168,12 +228,7 @@ class Engine final : public EngineBase {
       cudaError_t e = enqueue_post(C);
       if (e != cudaSuccess) return e;
     }
-    const int tok = C.group_begin(kGroupForces);
-    k_step_end<<<grid_for(C.ntanks, 128), 128, 0, C.stream>>>(
-        C.d_dt, C.d_dt_last, C.d_time, C.d_err, C.ntanks);
-    C.launches += 1;
-    C.group_end(tok);
-    return cudaGetLastError();
+    return step_end(C);
   }
 
   cudaError_t enqueue_prepare(Context& C) override {
@@ -307,10 +362,168 @@ class Engine final : public EngineBase {
     a.carry = 0;
     a.mode = kPassRK;
     a.walls_keep = 0;
+    a.stop = C.d_err + 1;
     return a;
   }
 
-  cudaError_t reorder(Context& C, const StageArgs<D, F>& a) {
+  cudaError_t step_end(Context& C) {
+    const int tok = C.group_begin(kGroupForces);
+    k_step_end<<<grid_for(C.ntanks, 128), 128, 0, C.stream>>>(
+        C.d_dt, C.d_dt_last, C.d_time, C.d_vmax, C.d_err, C.ntanks);
+    C.launches += 1;
+    C.group_end(tok);
+    return cudaGetLastError();
+  }
+
+  void release_lists(Context& C) {
+    C.release(C.d_list);
+    C.release(C.d_list_cnt);
+    C.d_list = nullptr;
+    C.d_list_cnt = nullptr;
+  }
+
+  // One step on neighbour lists (pairlist.cuh): one sort, lists for its
+  // stages, and per stage the wall pass and the pair sums.
+  cudaError_t enqueue_list_step(Context& C) {
+    cudaError_t e = enqueue_sort(C);
+    if (e != cudaSuccess) return e;
+    ListArgs<D, F> A{};
+    A.S = args(C, 0);
+    const StageArgs<D, F>& S = A.S;
+    A.pos_in = reinterpret_cast<typename ListArgs<D, F>::PosRec*>(posrec_);
+    A.dat_in = datrec_;
+    for (int k = 0; k < D; ++k) A.pin[k] = Y_.pos[k];
+    // Read by the list build only, before the first stage writes these.
+    A.lrec = reinterpret_cast<float4*>(datrec_b_);
+    A.list = C.d_list;
+    A.cnt = C.d_list_cnt;
+    // The face passes need the current cells; the sort's payload buffer that
+    // does not hold the permutation is free after the gather, and so is the
+    // permutation.
+    A.curkey = S.fc.on ? (C.perm == C.vals_a ? C.vals_b : C.vals_a) : nullptr;
+    A.vmax = C.d_vmax;
+    A.stop = C.d_err + 1;
+    A.n_walls = C.n_wall;
+    A.cap = C.list_cap;
+    A.margin = C.list_margin;
+    int tok = C.group_begin(kGroupReorder);
+    e = clear_wall_counts(C, S);
+    if (e != cudaSuccess) return e;
+    k_list_gather<D, F><<<grid_for(C.n, 256), 256, 0, C.stream>>>(A);
+    C.launches += 1;
+    C.group_end(tok);
+    tok = C.group_begin(kGroupSort);
+    if (C.n_wall > 0 && S.fbox != nullptr) {
+      k_list_select<D, F><<<grid_for(C.n_wall, 256), 256, 0, C.stream>>>(A);
+      C.launches += 1;
+    }
+    const int team = list_team(C);
+    if (team == 16) {
+      launch_build<16>(C, A);
+    } else if (team == 4) {
+      launch_build<4>(C, A);
+    } else {
+      launch_build<1>(C, A);
+    }
+    C.group_end(tok);
+    static const double w3[3] = {1.0, 1.0 / 4.0, 2.0 / 3.0};
+    static const double w2[2] = {1.0, 1.0 / 2.0};
+    const int stages = C.P.integrator == TG_SSPRK2 ? 2 : 3;
+    for (int s = 0; s < stages; ++s) {
+      A.first = s == 0;
+      A.last = s == stages - 1;
+      A.S.lincomb = s > 0;
+      A.S.w_new = (stages == 2 ? w2 : w3)[s];
+      A.pos_out = reinterpret_cast<typename ListArgs<D, F>::PosRec*>(s == 0 ? posrec_b_ : posrec_);
+      A.dat_out = s == 0 ? datrec_b_ : datrec_;
+      for (int k = 0; k < D; ++k) A.pout[k] = U_[s & 1].pos[k];
+      if (C.n_wall > 0) {
+        tok = C.group_begin(kGroupWalls);
+        StageArgs<D, F> a = A.S;  // the face passes' view of this stage
+        for (int k = 0; k < D; ++k) a.Y.pos[k] = A.pin[k];
+        a.datrec = A.dat_in;
+        if (s > 0 && a.fc.on) a.skey = A.curkey;
+        enqueue_gamma(C, a);
+        launch_list_walls(C, A);
+        if (a.fc.on) {
+          with_face_real(C, [&](auto real) {
+            k_face_terms<D, K, F, decltype(real)><<<face_grid(C), 128, 0, C.stream>>>(a);
+          });
+          C.launches += 1;
+        }
+        C.group_end(tok);
+      }
+      tok = C.group_begin(kGroupForces);
+      if constexpr (F == TG_FP32C) {
+        const int phys = physics_preset(C.P);
+        if (phys == kPhysTextbook) {
+          launch_list_forces<kPhysTextbook>(C, A, team);
+        } else if (phys == kPhysReference) {
+          launch_list_forces<kPhysReference>(C, A, team);
+        } else {
+          launch_list_forces<kPhysGeneric>(C, A, team);
+        }
+      } else {
+        launch_list_forces<kPhysGeneric>(C, A, team);
+      }
+      C.group_end(tok);
+      A.pos_in = A.pos_out;
+      A.dat_in = A.dat_out;
+      for (int k = 0; k < D; ++k) A.pin[k] = A.pout[k];
+    }
+    C.keys_valid = true;
+    C.order_valid = true;
+    if (C.P.post_integrate == TG_POST_SHIFTING) {
+      e = enqueue_post(C);
+      if (e != cudaSuccess) return e;
+    }
+    return step_end(C);
+  }
+
+  // Lanes per target of the list passes: one where the particles alone give
+  // every multiprocessor 16 warps, more for smaller runs (4 entries of the
+  // list per lane and turn, so 16 lanes take a 2D list at once).  A launch
+  // shape that asks for several lanes gets at least 4.
+  static int list_team(const Context& C) {
+    const int64_t full = 512 * static_cast<int64_t>(C.sm_count > 0 ? C.sm_count : 152);
+    if (4 * C.n_fluid < full) return 16;
+    return C.n_fluid < full || C.force_team > 1 ? 4 : 1;
+  }
+  template<int Team>
+  void launch_build(Context& C, const ListArgs<D, F>& A) {
+    const unsigned fluid = grid_for(C.n * Team, 128);
+    const int64_t cap = 8 * static_cast<int64_t>(C.sm_count > 0 ? C.sm_count : 152);
+    const unsigned walls = C.n_wall > 0 ? static_cast<unsigned>(std::min<int64_t>(
+                                              grid_for(C.n_wall * Team, 128), cap))
+                                        : 0u;
+    k_list_build<D, F, Team><<<fluid + walls, 128, 0, C.stream>>>(A, fluid);
+    C.launches += 1;
+  }
+  void launch_list_walls(Context& C, const ListArgs<D, F>& A) {
+    const int64_t cap = 16 * static_cast<int64_t>(C.sm_count > 0 ? C.sm_count : 152);
+    const unsigned grid =
+        static_cast<unsigned>(std::min<int64_t>(grid_for(C.n_wall * kListWallTeam, 128), cap));
+    k_list_walls<D, F, K><<<grid, 128, 0, C.stream>>>(A);
+    C.launches += 1;
+  }
+  template<int Phys>
+  void launch_list_forces(Context& C, const ListArgs<D, F>& A, int team) {
+    const int block = std::min(C.force_block, 128);
+    const size_t smem =
+        F == TG_FP32C ? sizeof(uint32_t) * kBandCap * static_cast<size_t>(block) : 0;
+    const unsigned grid = grid_for(C.n * team, block);
+    if (team == 16) {
+      k_list_forces<D, F, K, Phys, 16><<<grid, block, smem, C.stream>>>(A);
+    } else if (team == 4) {
+      k_list_forces<D, F, K, Phys, 4><<<grid, block, smem, C.stream>>>(A);
+    } else {
+      k_list_forces<D, F, K, Phys, 1><<<grid, block, smem, C.stream>>>(A);
+    }
+    C.launches += 1;
+  }
+
+  // Zero wall counts and empty fluid boxes for a gather.
+  static cudaError_t clear_wall_counts(Context& C, const StageArgs<D, F>& a) {
     cudaError_t e = cudaMemsetAsync(C.d_wall_count, 0, 2 * sizeof(uint32_t), C.stream);
     if (e != cudaSuccess) return e;
     if (a.fbox != nullptr) {
@@ -320,8 +533,13 @@ class Engine final : public EngineBase {
       if (e == cudaSuccess) {
         e = cudaMemsetAsync(C.d_fbox + 3 * C.ntanks, 0, half, C.stream);
       }
-      if (e != cudaSuccess) return e;
     }
+    return e;
+  }
+
+  cudaError_t reorder(Context& C, const StageArgs<D, F>& a) {
+    const cudaError_t e = clear_wall_counts(C, a);
+    if (e != cudaSuccess) return e;
     k_reorder<D, F><<<grid_for(C.n, 256), 256, 0, C.stream>>>(a);
     C.launches += 1;
     return cudaGetLastError();
@@ -339,7 +557,7 @@ class Engine final : public EngineBase {
     const int tok = C.group_begin(kGroupSort);
     if (C.order_valid && C.P.resort != 0) {
       e = near_sort(C.keys_a, X_.pkey, C.n, C.key_bits, C.keys_b, C.vals_b,
-                    C.near_scratch, C.stream, &C.launches);
+                    C.near_scratch, C.stream, &C.launches, C.d_err + 1);
       if (e != cudaSuccess) return e;
       C.sorted_keys = C.keys_b;
       C.perm = C.vals_b;
@@ -352,7 +570,8 @@ class Engine final : public EngineBase {
       C.perm = in_b ? C.vals_b : C.vals_a;
     }
     e = build_cell_table_fill(C.sorted_keys, C.n, C.total_keys, C.cell_start,
-                              C.cell_scratch, C.sm_count, C.stream, &C.launches);
+                              C.cell_scratch, C.sm_count, C.stream, &C.launches,
+                              C.d_err + 1);
     C.group_end(tok);
     return e;
   }
@@ -542,6 +761,8 @@ class Engine final : public EngineBase {
   PostArgs<D, F> post_{};
   PosRec* posrec_ = nullptr;
   DatRec* datrec_ = nullptr;
+  PosRec* posrec_b_ = nullptr;  // the list step's second records
+  DatRec* datrec_b_ = nullptr;
 };
 
 template <int D, int F, int K>

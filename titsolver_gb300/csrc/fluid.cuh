@@ -154,6 +154,8 @@ struct StageArgs {
   int walls_keep;    // k_walls: keep the carried wall densities
   unsigned* fbox;     // per-tank fluid bounding box (k_reorder)
   FaceArgs fc;        // boundary faces (fc.on = 0: particle walls)
+  const uint32_t* stop;  // not zero: a step on neighbour lists has to be
+                         // repeated, and the kernels leave everything as it is
 };
 
 // Order-preserving map of floats to unsigned 32-bit integers (and back),
@@ -244,14 +246,14 @@ __device__ __forceinline__ void fold_fluid_box(unsigned* box, int ntanks,
   }
 }
 
-// True when no fluid particle of the tank can lie within the support radius
-// of a point with tank-local FP32 coordinates xl: its distance to the
-// tank's fluid bounding box exceeds R plus a margin that covers the FP32
-// rounding of both coordinates (wall_skip_r2_f), or the tank has no fluid
-// this stage.
+// True when no fluid particle of the tank can lie within reach of a point
+// with tank-local FP32 coordinates xl: its distance to the tank's fluid
+// bounding box exceeds the reach (the support radius plus a margin that
+// covers the FP32 rounding of both coordinates: wall_skip_r2_f, squared), or
+// the tank has no fluid this stage.
 template<int D>
 __device__ __forceinline__ bool beyond_fluid(const unsigned* box, int ntanks,
-                                             uint32_t tk, const TankDev& T,
+                                             uint32_t tk, float reach2,
                                              const float* xl) {
   if (box == nullptr) return false;  // no box this stage: walk every wall
   float g2 = 0.f;
@@ -263,7 +265,7 @@ __device__ __forceinline__ bool beyond_fluid(const unsigned* box, int ntanks,
     const float g = fmaxf(fmaxf(order_dec(elo) - xl[k], xl[k] - order_dec(ehi)), 0.f);
     g2 += g * g;
   }
-  return g2 > T.wall_skip_r2_f;
+  return g2 > reach2;
 }
 
 // Tank-local FP32 coordinates: from the FP64 position (FP64 form) or from
@@ -641,6 +643,7 @@ __device__ __forceinline__ void commit_wall(const StageArgs<D, F>& A, int64_t e,
 template<int D, int F>
 __global__ void __launch_bounds__(256) k_reorder(StageArgs<D, F> A) {
   using R = typename StageArgs<D, F>::R;
+  if (*A.stop != 0u) return;
   const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const bool valid = j < A.n;
   double dt_a = __longlong_as_double(0x7ff0000000000000ll);
@@ -829,6 +832,7 @@ constexpr int wall_team() {
 template<int D, int F>
 __global__ void __launch_bounds__(256)
     k_wall_select(StageArgs<D, F> A, int64_t n_walls) {
+  if (*A.stop != 0u) return;
   const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   bool act = false;
   uint32_t e = 0;
@@ -849,7 +853,7 @@ __global__ void __launch_bounds__(256)
       load_pos(A.posrec, e, oe);
       local_coords<D>(T, c, oe, xl);
     }
-    act = !beyond_fluid<D>(A.fbox, A.ntanks, tk, T, xl);
+    act = !beyond_fluid<D>(A.fbox, A.ntanks, tk, T.wall_skip_r2_f, xl);
   }
   // One atomic per warp.
   const unsigned mask = __ballot_sync(0xffffffffu, act);
@@ -1138,6 +1142,57 @@ struct PairF32 {
   }
 };
 
+// Home state of the fluid particle at cell-order slot i: its new state, and
+// the cell key (and FP32 offset) of the new position; c is its cell in the
+// order of this sort.
+template<int D, int F>
+__device__ __forceinline__ void commit_fluid(
+    const StageArgs<D, F>& A, int64_t i, uint32_t id, const TankDev& T, const int* c,
+    const double* pn, const typename StageArgs<D, F>::R* vn,
+    typename StageArgs<D, F>::R rn, const typename StageArgs<D, F>::R* dv,
+    typename StageArgs<D, F>::R drho) {
+  int cn[3] = {0, 0, 0};
+  if constexpr (F == TG_FP64) {
+    bool outside = false;
+    cell_of<D>(T, pn, cn, outside);
+    if (outside) atomicOr(A.err, static_cast<uint32_t>(TG_DEV_OUTSIDE_GRID));
+  } else {
+    // Offset from the old cell corner (exact FP64 difference, rounded once),
+    // then a shift by whole cells in FP32, clamped at the grid border.
+    bool outside = false;
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      const float o = __double2float_rn(
+          pn[k] - fma(static_cast<double>(c[k]), T.cs, T.lo[k]));
+      const float f = floorf(__fdividef(o, T.cs_f));
+      int ck = c[k] + (isfinite(f) ? static_cast<int>(f) : 0);
+      if (ck < 0 || ck >= T.nc[k]) {
+        outside = true;
+        ck = min(max(ck, 0), T.nc[k] - 1);
+      }
+      cn[k] = ck;
+      A.X.off[k][i] = o - static_cast<float>(ck - c[k]) * T.cs_f;
+    }
+    if (outside) atomicOr(A.err, static_cast<uint32_t>(TG_DEV_OUTSIDE_GRID));
+  }
+  A.X.pkey[i] = A.skey[i];  // read before the key write: the buffers may alias
+  A.X.key[i] = key_of(flat_cell<D>(T, cn), false);
+  bool finite = true;
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    A.X.pos[k][i] = pn[k];
+    A.X.vel[k][i] = vn[k];
+    A.X.dv[k][i] = dv[k];
+    finite = finite && finite_bits(pn[k]) && isfinite(vn[k]);
+  }
+  A.X.rho[i] = rn;
+  A.X.drho[i] = drho;
+  A.X.id[i] = id;
+  if (!(finite && isfinite(rn))) {
+    atomicOr(A.err, static_cast<uint32_t>(TG_DEV_NONFINITE_STATE));
+  }
+}
+
 // Euler update (time_integrator.hpp:203-207), SSPRK lincomb (:212-223) and
 // the cell key (and FP32 offset) of the new position; positions in FP64,
 // the rest in the form's type.
@@ -1210,46 +1265,7 @@ __device__ __forceinline__ void forces_epilogue(
     }
     rn = w0r * A.Udst.rho[i] + wr * rn;
   }
-  int cn[3] = {0, 0, 0};
-  if constexpr (F == TG_FP64) {
-    bool outside = false;
-    cell_of<D>(T, pn, cn, outside);
-    if (outside) atomicOr(A.err, static_cast<uint32_t>(TG_DEV_OUTSIDE_GRID));
-  } else {
-    // Offset from the old cell corner (exact FP64 difference, rounded once),
-    // then a shift by whole cells in FP32, clamped at the grid border.
-    bool outside = false;
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-      const float o = __double2float_rn(
-          pn[k] - fma(static_cast<double>(c[k]), T.cs, T.lo[k]));
-      const float f = floorf(__fdividef(o, T.cs_f));
-      int ck = c[k] + (isfinite(f) ? static_cast<int>(f) : 0);
-      if (ck < 0 || ck >= T.nc[k]) {
-        outside = true;
-        ck = min(max(ck, 0), T.nc[k] - 1);
-      }
-      cn[k] = ck;
-      A.X.off[k][i] = o - static_cast<float>(ck - c[k]) * T.cs_f;
-    }
-    if (outside) atomicOr(A.err, static_cast<uint32_t>(TG_DEV_OUTSIDE_GRID));
-  }
-  A.X.pkey[i] = A.skey[i];  // read before the key write: the buffers may alias
-  A.X.key[i] = key_of(flat_cell<D>(T, cn), false);
-  bool finite = true;
-#pragma unroll
-  for (int k = 0; k < D; ++k) {
-    A.X.pos[k][i] = pn[k];
-    A.X.vel[k][i] = vn[k];
-    A.X.dv[k][i] = dv_keep[k];
-    finite = finite && finite_bits(pn[k]) && isfinite(vn[k]);
-  }
-  A.X.rho[i] = rn;
-  A.X.drho[i] = drho_keep;
-  A.X.id[i] = id;
-  if (!(finite && isfinite(rn))) {
-    atomicOr(A.err, static_cast<uint32_t>(TG_DEV_NONFINITE_STATE));
-  }
+  commit_fluid<D, F>(A, i, id, T, c, pn, vn, rn, dv_keep, drho_keep);
 }
 
 // Face boundaries (fluid_equations.hpp:241-247, 276-292): per adjacent face
@@ -2125,6 +2141,7 @@ __global__ void __launch_bounds__(128) k_sumdens(CloudArgs<D> A) {
 // sums.
 template<int D, int F>
 __global__ void __launch_bounds__(128) k_gamma_init(StageArgs<D, F> A) {
+  if (*A.stop != 0u) return;
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= A.n) return;
   const FaceArgs& fc = A.fc;
@@ -2371,13 +2388,19 @@ __global__ void __launch_bounds__(256)
   if (drho != nullptr) drho[id] = X.drho[i];
 }
 
-// End of step: advance per-tank time, keep dt, reset the dt reduction.
-static __global__ void k_step_end(double* dt, double* dt_last, double* time,
-                                  uint32_t* err, int ntanks) {
+// End of step: advance per-tank time, keep dt, reset the reductions, count
+// the step.  status: the error word, the stop word, the steps finished; a
+// stopped step advances nothing.
+static __global__ void k_step_end(double* dt, double* dt_last, double* time, unsigned* vmax,
+                                  uint32_t* status, int ntanks) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool done = status[1] == 0u;
+  if (t == 0 && done) status[2] += 1u;
   if (t >= ntanks) return;
+  uint32_t* err = status;
+  vmax[t] = 0u;
   const double d = dt[t];
-  if (isfinite(d)) {
+  if (done && isfinite(d)) {
     if (!(d > 0.0)) atomicOr(err, static_cast<uint32_t>(TG_DEV_BAD_DT));
     time[t] += d;
     dt_last[t] = d;

@@ -137,7 +137,7 @@ __device__ __forceinline__ bool post_target(const PostArgs<D, F>& A, int64_t& i,
                                             uint32_t& id, const TankDev*& T,
                                             int* c) {
   i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= A.S.n) return false;
+  if (i >= A.S.n || *A.S.stop != 0u) return false;
   id = A.S.Y.id[i];
   const uint32_t key = A.S.skey[i];
   T = &A.S.tanks[tank_of_key(key, A.S.tank_off, A.S.ntanks)];

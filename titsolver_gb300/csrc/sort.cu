@@ -282,7 +282,8 @@ struct FillRun {
 __global__ void __launch_bounds__(256)
     k_fill_starts(const uint32_t* __restrict__ keys, int64_t n, uint32_t total_keys,
                   uint32_t* __restrict__ cell_start, FillRun* __restrict__ runs,
-                  uint32_t* __restrict__ run_count) {
+                  uint32_t* __restrict__ run_count, const uint32_t* __restrict__ stop) {
+  if (stop != nullptr && *stop != 0u) return;
   const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   // Every lane reaches the vote below, the ones past n with an empty run.
@@ -340,13 +341,13 @@ size_t cell_fill_scratch_bytes(uint32_t total_keys) {
 cudaError_t build_cell_table_fill(const uint32_t* sorted_keys, int64_t n,
                                   uint32_t total_keys, uint32_t* cell_start,
                                   void* scratch, int sm_count, cudaStream_t stream,
-                                  int64_t* launches) {
+                                  int64_t* launches, const uint32_t* stop) {
   auto* count = static_cast<uint32_t*>(scratch);
   auto* runs = reinterpret_cast<FillRun*>(static_cast<unsigned char*>(scratch) + 256);
   cudaError_t e = cudaMemsetAsync(count, 0, sizeof(uint32_t), stream);
   if (e != cudaSuccess) return e;
   k_fill_starts<<<static_cast<unsigned>((n + 1 + 255) / 256), 256, 0, stream>>>(
-      sorted_keys, n, total_keys, cell_start, runs, count);
+      sorted_keys, n, total_keys, cell_start, runs, count, stop);
   k_fill_runs<<<static_cast<unsigned>(8 * (sm_count > 0 ? sm_count : 152)), 256, 0, stream>>>(
       cell_start, runs, count);
   *launches += 2;

@@ -42,12 +42,13 @@ cudaError_t radix_sort(uint32_t* keys_a, uint32_t* vals_a, uint32_t* keys_b,
 // the sorted keys, out_perm the slot of each.  Four kernels and the movers'
 // radix passes.  The scratch holds a completion counter that must be zero
 // before the first near_sort (near_sort_reset; every near_sort leaves it
-// zero).
+// zero).  With stop, nothing is sorted while *stop is not zero.
 size_t near_sort_scratch_bytes(int64_t n);
 cudaError_t near_sort_reset(void* scratch, int64_t n, cudaStream_t stream);
 cudaError_t near_sort(const uint32_t* keys, const uint32_t* prev, int64_t n,
                       int key_bits, uint32_t* out_keys, uint32_t* out_perm,
-                      void* scratch, cudaStream_t stream, int64_t* launches);
+                      void* scratch, cudaStream_t stream, int64_t* launches,
+                      const uint32_t* stop = nullptr);
 
 // cell_start[c] = first sorted index whose key >= c, for c in
 // [0, total_cells]; cell_start[total_cells] = n.  Every cell searches the
@@ -63,11 +64,11 @@ cudaError_t build_cell_table(const uint32_t* sorted_keys, int64_t n,
 // the starts of the cells between its key and the previous one, and long
 // empty stretches are filled by whole blocks from a list.  Writes each entry
 // once; the scratch holds that list (cell_fill_scratch_bytes).  A memset and
-// two kernels.
+// two kernels.  With stop, nothing is written while *stop is not zero.
 size_t cell_fill_scratch_bytes(uint32_t total_keys);
 cudaError_t build_cell_table_fill(const uint32_t* sorted_keys, int64_t n,
                                   uint32_t total_keys, uint32_t* cell_start,
                                   void* scratch, int sm_count, cudaStream_t stream,
-                                  int64_t* launches);
+                                  int64_t* launches, const uint32_t* stop = nullptr);
 
 }  // namespace tg

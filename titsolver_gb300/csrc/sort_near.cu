@@ -74,7 +74,12 @@ __global__ void __launch_bounds__(kScanBlock)
     k_ns_flags_scan(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ prev,
                     int64_t n, int64_t nwords, int64_t nblocks, uint32_t* __restrict__ mask,
                     uint32_t* __restrict__ prefix, uint32_t* bsum, uint32_t* __restrict__ total,
-                    uint32_t* done) {
+                    uint32_t* done, const uint32_t* __restrict__ stop) {
+  if (stop != nullptr && *stop != 0u) {
+    // No movers: the kernels that read the count have nothing to do.
+    if (blockIdx.x == 0 && threadIdx.x == 0) *total = 0u;
+    return;
+  }
   __shared__ uint32_t s_warp[32];
   __shared__ uint32_t s_last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -140,7 +145,8 @@ __global__ void __launch_bounds__(kNsBlock)
     k_ns_compact(const uint32_t* __restrict__ keys, int64_t n,
                  const uint32_t* __restrict__ mask, const uint32_t* __restrict__ prefix,
                  const uint32_t* __restrict__ bsum, uint32_t* __restrict__ mkey,
-                 uint32_t* __restrict__ mslot) {
+                 uint32_t* __restrict__ mslot, const uint32_t* __restrict__ stop) {
+  if (stop != nullptr && *stop != 0u) return;
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int64_t w = i >> 5;
@@ -182,7 +188,9 @@ __global__ void __launch_bounds__(kNsBlock)
                  const uint32_t* __restrict__ mask, const uint32_t* __restrict__ prefix,
                  const uint32_t* __restrict__ bsum, const uint32_t* __restrict__ total,
                  const uint32_t* __restrict__ mkey, const uint32_t* __restrict__ mslot,
-                 uint32_t* __restrict__ out_keys, uint32_t* __restrict__ out_perm) {
+                 uint32_t* __restrict__ out_keys, uint32_t* __restrict__ out_perm,
+                 const uint32_t* __restrict__ stop) {
+  if (stop != nullptr && *stop != 0u) return;
   __shared__ uint32_t s_key[kMoverWindow], s_slot[kMoverWindow];
   __shared__ uint32_t s_lo, s_hi;
   const int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x;
@@ -324,7 +332,8 @@ cudaError_t near_sort_reset(void* scratch, int64_t n, cudaStream_t stream) {
 
 cudaError_t near_sort(const uint32_t* keys, const uint32_t* prev, int64_t n,
                       int key_bits, uint32_t* out_keys, uint32_t* out_perm,
-                      void* scratch, cudaStream_t stream, int64_t* launches) {
+                      void* scratch, cudaStream_t stream, int64_t* launches,
+                      const uint32_t* stop) {
   if (n <= 0) return cudaSuccess;
   const NearLayout L = near_layout(n);
   auto* base = static_cast<unsigned char*>(scratch);
@@ -339,8 +348,9 @@ cudaError_t near_sort(const uint32_t* keys, const uint32_t* prev, int64_t n,
   auto* ms1 = reinterpret_cast<uint32_t*>(base + L.off_ms1);
   const unsigned gslots = static_cast<unsigned>((n + kNsBlock - 1) / kNsBlock);
   k_ns_flags_scan<<<static_cast<unsigned>(L.nblocks), kScanBlock, 0, stream>>>(
-      keys, prev, n, L.nwords, L.nblocks, mask, prefix, bsum, total, done);
-  k_ns_compact<<<gslots, kNsBlock, 0, stream>>>(keys, n, mask, prefix, bsum, mk0, ms0);
+      keys, prev, n, L.nwords, L.nblocks, mask, prefix, bsum, total, done, stop);
+  k_ns_compact<<<gslots, kNsBlock, 0, stream>>>(keys, n, mask, prefix, bsum, mk0, ms0,
+                                                 stop);
   *launches += 2;
   bool in_b = false;
   cudaError_t e = radix_sort(mk0, ms0, mk1, ms1, n, key_bits, false, base + L.off_radix,
@@ -349,7 +359,7 @@ cudaError_t near_sort(const uint32_t* keys, const uint32_t* prev, int64_t n,
   const uint32_t* mkey = in_b ? mk1 : mk0;
   const uint32_t* mslot = in_b ? ms1 : ms0;
   k_ns_stayers<<<gslots, kNsBlock, 0, stream>>>(prev, n, mask, prefix, bsum, total, mkey,
-                                                 mslot, out_keys, out_perm);
+                                                 mslot, out_keys, out_perm, stop);
   k_ns_movers<<<1216, kNsBlock, 0, stream>>>(prev, n, mask, prefix, bsum, L.nwords, total,
                                              mkey, mslot, out_keys, out_perm);
   *launches += 2;
