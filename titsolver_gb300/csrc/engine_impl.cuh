@@ -157,7 +157,8 @@ class Engine final : public EngineBase {
         e = C.alloc(reinterpret_cast<void**>(&C.d_list_cnt), sizeof(uint32_t) * C.n);
       }
       if (e == cudaSuccess && datrec_b_ == nullptr) {
-        e = C.alloc(reinterpret_cast<void**>(&datrec_b_), sizeof(DatRec) * C.n);
+        // The list build reads a few 16-byte records past the last.
+        e = C.alloc(reinterpret_cast<void**>(&datrec_b_), sizeof(DatRec) * (C.n + kListScan));
         if (e == cudaSuccess && F == TG_FP64) {
           e = C.alloc(reinterpret_cast<void**>(&posrec_b_), sizeof(PosRec) * C.n);
         }
@@ -434,6 +435,9 @@ class Engine final : public EngineBase {
       A.last = s == stages - 1;
       A.S.lincomb = s > 0;
       A.S.w_new = (stages == 2 ? w2 : w3)[s];
+      A.w0 = 1.0 - A.S.w_new;
+      A.wr = static_cast<R>(A.S.w_new);
+      A.w0r = static_cast<R>(A.w0);
       A.pos_out = reinterpret_cast<typename ListArgs<D, F>::PosRec*>(s == 0 ? posrec_b_ : posrec_);
       A.dat_out = s == 0 ? datrec_b_ : datrec_;
       for (int k = 0; k < D; ++k) A.pout[k] = U_[s & 1].pos[k];

@@ -509,8 +509,8 @@ __device__ __forceinline__ float dist2_exact(const float* a, const float* b,
 // s2_f comes from cell-relative offsets, each rounded once from an exact
 // FP64 difference.  With u = 2^-24, offsets within a cell size cs (plus a
 // few ulps) of their cell corner and the candidate's cell within k cells of
-// the target's (cs = R / k), each FP32 component of r_ab is within
-// (3k + 3) u cs + u |r_ab| <= 7 u R of the exact one (the FP64 cell corners
+// the target's (cs = 1.05 R / k), each FP32 component of r_ab is within
+// (3k + 3) u cs + u |r_ab| < 8 u R of the exact one (the FP64 cell corners
 // add 2^-52 of the coordinates, negligible within 2^20 cells of the
 // origin), so |s2_f - s2| < 32 u R^2: far inside the band R^2 (1 -+ 2^-14)
 // = R^2 (1 -+ 1024 u).  Below the band the pair is a neighbour, above it is

@@ -63,6 +63,8 @@ struct ListArgs {
   int cap;                // entries per slot, a multiple of 4
   float margin;           // acceleration share of delta, in R
   int first, last;
+  double w0;              // 1 - S.w_new, and both in the form's type
+  R w0r, wr;
 };
 
 // Entry p of slot s.
@@ -74,9 +76,8 @@ __device__ __forceinline__ size_t list_at(int64_t s, uint32_t p, int cap) {
 // The displacement bound of a tank's particles in this step.
 template<int D, int F>
 __device__ __forceinline__ float list_delta(const ListArgs<D, F>& A, const TankDev& T,
-                                            uint32_t tk) {
-  const float d = static_cast<float>(A.S.dt[tk]) * __uint_as_float(A.vmax[tk]) * 1.0001f +
-                  A.margin * T.R_f;
+                                            uint32_t tk, float dt) {
+  const float d = dt * __uint_as_float(A.vmax[tk]) * 1.0001f + A.margin * T.R_f;
   return fminf(d, 0.25f * T.R_f);  // also for a tank without fluid (dt = inf)
 }
 
@@ -265,7 +266,8 @@ __global__ void __launch_bounds__(256) k_list_select(ListArgs<D, F> A) {
     const TankDev& T = S.tanks[tk];
     const float4 x = A.lrec[e];
     const float xl[3] = {x.x, x.y, x.z};
-    const float reach = sqrtf(T.wall_skip_r2_f) + 2.f * list_delta(A, T, tk);
+    const float reach = sqrtf(T.wall_skip_r2_f) +
+                        2.f * list_delta(A, T, tk, static_cast<float>(S.dt[tk]));
     act = !beyond_fluid<D>(S.fbox, S.ntanks, tk, reach * reach, xl);
   }
   const unsigned mask = __ballot_sync(0xffffffffu, act);
@@ -288,6 +290,7 @@ __global__ void __launch_bounds__(256) k_list_select(ListArgs<D, F> A) {
 
 struct ListRows {
   int y0, y1, z0, z1, x0, x1;  // the block of cells
+  int yb, zb, span;            // its unclipped corner and width
   float RL, RL2;
   bool border;
 };
@@ -303,6 +306,9 @@ __device__ __forceinline__ ListRows list_rows(const TankDev& T, const int* c, co
   W.border = c[0] - kk <= 0 || c[0] + kk >= T.nc[0] - 1 || c[1] - kk <= 0 ||
              c[1] + kk >= T.nc[1] - 1;
   if constexpr (D == 3) W.border = W.border || c[2] - kk <= 0 || c[2] + kk >= T.nc[2] - 1;
+  W.yb = c[1] - kk;
+  W.zb = D == 3 ? c[2] - kk : 0;
+  W.span = 2 * kk + 1;
   W.x0 = max(c[0] - kk, 0);
   W.x1 = min(c[0] + kk, T.nc[0] - 1);
   W.y0 = max(c[1] - kk, 0);
@@ -368,6 +374,15 @@ __device__ __forceinline__ bool list_near_fp64(double* const* pos, int64_t a, ui
   return s <= RL * RL;
 }
 
+// Candidates loaded together, and 128-thread blocks per SM: the build waits
+// for its loads, so warps count most.  Measured sort + build per step, 3D 2M
+// / 2D 1.28M fluid particles, in ms (candidates x blocks): 2 x 12 1.03 / .338
+// (2 x 8 1.15 / .358, 2 x 10 1.07 / .341, 2 x 16 1.08 / .358, 1 x 16 1.07 /
+// .363, 4 x 8 1.10 / .347, 4 x 12 1.25 / .343); loading one record ahead of
+// the test instead 1.23 / .385.
+constexpr uint32_t kListScan = 2;
+constexpr int kListBuildBlocks = 12;
+
 // Appends accepted entries to a list in groups of four.
 struct ListWriter {
   uint4* out;
@@ -390,15 +405,14 @@ struct ListWriter {
 };
 
 // The list of slot i, by Team lanes (lane tl of the team; the lanes split
-// the rows).  wall_target: fluid entries only.  A warp with a border target
+// the rows).  Wall targets list fluid entries only.  A warp with a border target
 // takes the FP64 test for all its targets: kept apart, so that the common
 // loop holds no FP64 instruction (selected per candidate, they issued for
 // every candidate and the build of 2M particles took 9.2 ms).
-template<int D, int F, int Team, bool Border>
+template<int D, int F, int Team, bool Wall, bool Border>
 __device__ __forceinline__ void build_list(const ListArgs<D, F>& A, const TankDev& T,
                                            const ListRows& W, const float* xl, int64_t i,
-                                           bool target, bool wall_target, int tl,
-                                           unsigned tmask) {
+                                           bool target, int tl, unsigned tmask) {
   const StageArgs<D, F>& S = A.S;
   const uint32_t ia = static_cast<uint32_t>(i);
   const auto accept = [&](const float4& b, uint32_t j) {
@@ -414,7 +428,7 @@ __device__ __forceinline__ void build_list(const ListArgs<D, F>& A, const TankDe
     } else {
       near = list_near_fp64<D>(S.Y.pos, i, j, static_cast<double>(W.RL));
     }
-    return near && j != ia && !(wall_target && b.w < 0.f);
+    return near && j != ia && !(Wall && b.w < 0.f);
   };
   const uint32_t cap = static_cast<uint32_t>(A.cap);
   uint32_t cnt = 0;
@@ -422,16 +436,25 @@ __device__ __forceinline__ void build_list(const ListArgs<D, F>& A, const TankDe
     ListWriter w;
     w.out = reinterpret_cast<uint4*>(A.list) + (list_at(i, 0, A.cap) >> 2);
     w.cap = cap;
-    for (int z = W.z0; z <= W.z1; ++z) {
-      for (int y = W.y0; y <= W.y1; ++y) {
-        uint32_t s, e;
-        list_row<D>(T, W, xl, S.cell_start, y, z, s, e);
-        float4 bn = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (s < e) bn = A.lrec[s];
-        for (uint32_t j = s; j < e; ++j) {
-          const float4 b = bn;
-          if (j + 1 < e) bn = A.lrec[j + 1];
-          if (accept(b, j)) w.add(j);
+    // Every lane takes its rows by their offset from its own cell's row (out
+    // of reach or not), so that the lanes of a row of cells, most of a warp,
+    // walk the same rows together.
+    for (int z = W.zb; z < W.zb + (D == 3 ? W.span : 1); ++z) {
+      for (int y = W.yb; y < W.yb + W.span; ++y) {
+        uint32_t s = 0, e = 0;
+        if (y >= W.y0 && y <= W.y1 && z >= W.z0 && z <= W.z1) {
+          list_row<D>(T, W, xl, S.cell_start, y, z, s, e);
+        }
+        // Batches of candidates in flight; lrec is readable kListScan - 1
+        // records past the last.
+        for (uint32_t j = s; j < e; j += kListScan) {
+          float4 b[kListScan];
+#pragma unroll
+          for (uint32_t q = 0; q < kListScan; ++q) b[q] = A.lrec[j + q];
+#pragma unroll
+          for (uint32_t q = 0; q < kListScan; ++q) {
+            if (j + q < e && accept(b[q], j + q)) w.add(j + q);
+          }
         }
       }
     }
@@ -465,12 +488,12 @@ __device__ __forceinline__ void build_list(const ListArgs<D, F>& A, const TankDe
 }
 
 // Called by whole warps; lanes without a target take part in the votes.
-template<int D, int F, int Team>
+template<int D, int F, int Team, bool Wall>
 __device__ __forceinline__ void build_lists(const ListArgs<D, F>& A, int64_t i, bool target,
-                                            bool wall_target, int tl, unsigned tmask) {
+                                            int tl, unsigned tmask) {
   const StageArgs<D, F>& S = A.S;
   const TankDev* T = S.tanks;
-  ListRows W{0, -1, 0, -1, 0, 0, 0.f, 0.f, false};
+  ListRows W{0, -1, 0, -1, 0, 0, 0, 0, 0, 0.f, 0.f, false};
   float xl[3] = {0.f, 0.f, 0.f};
   if (target) {
     const uint32_t key = S.skey[i];
@@ -482,19 +505,20 @@ __device__ __forceinline__ void build_lists(const ListArgs<D, F>& A, int64_t i, 
     xl[0] = x.x;
     xl[1] = x.y;
     xl[2] = x.z;
-    W = list_rows<D>(*T, c, xl, T->R_f + T->list_slack_f + 2.f * list_delta(A, *T, tk));
+    W = list_rows<D>(*T, c, xl, T->R_f + T->list_slack_f +
+                          2.f * list_delta(A, *T, tk, static_cast<float>(S.dt[tk])));
   }
   if (__any_sync(0xffffffffu, W.border)) {
-    build_list<D, F, Team, true>(A, *T, W, xl, i, target, wall_target, tl, tmask);
+    build_list<D, F, Team, Wall, true>(A, *T, W, xl, i, target, tl, tmask);
   } else {
-    build_list<D, F, Team, false>(A, *T, W, xl, i, target, wall_target, tl, tmask);
+    build_list<D, F, Team, Wall, false>(A, *T, W, xl, i, target, tl, tmask);
   }
 }
 
 // Blocks below fluid_blocks take the slots in order (walls excepted), the
 // others the listed walls in turn.
 template<int D, int F, int Team>
-__global__ void __launch_bounds__(128) k_list_build(ListArgs<D, F> A, unsigned fluid_blocks) {
+__global__ void __launch_bounds__(128, kListBuildBlocks) k_list_build(ListArgs<D, F> A, unsigned fluid_blocks) {
   if (*A.stop != 0u) return;
   const StageArgs<D, F>& S = A.S;
   const int tl = Team == 1 ? 0 : static_cast<int>(threadIdx.x % Team);
@@ -503,7 +527,7 @@ __global__ void __launch_bounds__(128) k_list_build(ListArgs<D, F> A, unsigned f
     const int64_t i =
         (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / Team;
     const bool target = i < S.n && !(S.Y.id[i] & kWallBit);
-    build_lists<D, F, Team>(A, target ? i : 0, target, false, tl, tmask);
+    build_lists<D, F, Team, false>(A, target ? i : 0, target, tl, tmask);
     return;
   }
   const bool all = S.fbox == nullptr;
@@ -517,7 +541,7 @@ __global__ void __launch_bounds__(128) k_list_build(ListArgs<D, F> A, unsigned f
   for (int64_t w = w0; w < count; w += step) {
     const bool target = w + in_warp < count;
     const int64_t i = target ? walls[w + in_warp] : 0;
-    build_lists<D, F, Team>(A, i, target, true, tl, tmask);
+    build_lists<D, F, Team, true>(A, i, target, tl, tmask);
   }
 }
 
@@ -940,6 +964,7 @@ __device__ __forceinline__ void list_epilogue(const ListArgs<D, F>& A, int64_t i
   const StageArgs<D, F>& S = A.S;
   const double dt = S.dt[tk];
   const R dtr = static_cast<R>(dt);
+  const float dtf = static_cast<float>(dtr);
   double pn[3] = {0.0, 0.0, 0.0};
   R vn[3] = {R(0), R(0), R(0)};
 #pragma unroll
@@ -948,25 +973,33 @@ __device__ __forceinline__ void list_epilogue(const ListArgs<D, F>& A, int64_t i
     vn[k] = va[k] + dtr * dv[k];
   }
   R rn = rho_self + dtr * drho;
+  // The displacement since the step's start, for the bound: dt v in the
+  // first stage, so that the second starts from u_n + dt v_n and ends at
+  // w dt (v_n + v) from u_n (few FP64 operations: their pipe is what the
+  // compensated form's update is bound by).
+  float dis[3] = {0.f, 0.f, 0.f};
   if (S.lincomb) {
-    const double w = S.w_new, w0 = 1.0 - S.w_new;
-    const R wr = static_cast<R>(w), w0r = static_cast<R>(w0);
+    const R wr = A.wr, w0r = A.w0r;
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-      pn[k] = fma(w0, S.Y.pos[k][i], w * pn[k]);
-      vn[k] = w0r * S.Udst.vel[k][i] + wr * vn[k];
+      const R v0 = S.Udst.vel[k][i];
+      dis[k] = static_cast<float>(wr) * dtf * (static_cast<float>(v0) + static_cast<float>(va[k]));
+      pn[k] = fma(A.w0, S.Y.pos[k][i], S.w_new * pn[k]);
+      vn[k] = w0r * v0 + wr * vn[k];
     }
     rn = w0r * S.Udst.rho[i] + wr * rn;
+  } else {
+#pragma unroll
+    for (int k = 0; k < D; ++k) dis[k] = dtf * static_cast<float>(va[k]);
   }
   if (!A.last) {
     float d2 = 0.f;
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-      const float d = __double2float_rn(pn[k] - S.Y.pos[k][i]);
-      d2 = fmaf(d, d, d2);
+      d2 = fmaf(dis[k], dis[k], d2);
       A.pout[k][i] = pn[k];
     }
-    const float delta = list_delta(A, T, tk);
+    const float delta = list_delta(A, T, tk, dtf);
     if (!(d2 <= delta * delta)) atomicOr(A.stop, kStopMoved);
     if (A.curkey != nullptr) {
       int cn[3] = {0, 0, 0};
