@@ -8,6 +8,7 @@
 #include "fluid.cuh"
 #include "pairlist.cuh"
 #include "post.cuh"
+#include "postlist.cuh"
 #include "sort.cuh"
 
 namespace tg {
@@ -430,23 +431,22 @@ class Engine final : public EngineBase {
     static const double w3[3] = {1.0, 1.0 / 4.0, 2.0 / 3.0};
     static const double w2[2] = {1.0, 1.0 / 2.0};
     const int stages = C.P.integrator == TG_SSPRK2 ? 2 : 3;
+    const bool shifting = C.P.post_integrate == TG_POST_SHIFTING;
     for (int s = 0; s < stages; ++s) {
       A.first = s == 0;
-      A.last = s == stages - 1;
+      A.last = s == stages - 1 && !shifting;
+      A.post = s == stages - 1 && shifting;
       A.S.lincomb = s > 0;
       A.S.w_new = (stages == 2 ? w2 : w3)[s];
       A.w0 = 1.0 - A.S.w_new;
       A.wr = static_cast<R>(A.S.w_new);
       A.w0r = static_cast<R>(A.w0);
-      A.pos_out = reinterpret_cast<typename ListArgs<D, F>::PosRec*>(s == 0 ? posrec_b_ : posrec_);
-      A.dat_out = s == 0 ? datrec_b_ : datrec_;
+      A.pos_out = reinterpret_cast<typename ListArgs<D, F>::PosRec*>(s == 1 ? posrec_ : posrec_b_);
+      A.dat_out = s == 1 ? datrec_ : datrec_b_;
       for (int k = 0; k < D; ++k) A.pout[k] = U_[s & 1].pos[k];
       if (C.n_wall > 0) {
         tok = C.group_begin(kGroupWalls);
-        StageArgs<D, F> a = A.S;  // the face passes' view of this stage
-        for (int k = 0; k < D; ++k) a.Y.pos[k] = A.pin[k];
-        a.datrec = A.dat_in;
-        if (s > 0 && a.fc.on) a.skey = A.curkey;
+        const StageArgs<D, F> a = list_stage_view(A);
         enqueue_gamma(C, a);
         launch_list_walls(C, A);
         if (a.fc.on) {
@@ -475,13 +475,64 @@ class Engine final : public EngineBase {
       A.dat_in = A.dat_out;
       for (int k = 0; k < D; ++k) A.pin[k] = A.pout[k];
     }
+    if (shifting) {
+      tok = C.group_begin(kGroupPost);
+      A.first = 0;
+      A.last = 1;
+      A.post = 0;
+      ListPostArgs<D, F> q;
+      q.L = A;
+      q.P = post_args(C);
+      q.P.S = list_stage_view(A);
+      if (C.n_wall > 0) {
+        enqueue_gamma(C, q.P.S);
+        launch_list_walls(C, A);
+        if (C.faces.on) {
+          with_face_real(C, [&](auto real) {
+            k_post_faces<D, F, K, decltype(real)><<<face_grid(C), 128, 0, C.stream>>>(q.P);
+          });
+          C.launches += 1;
+        }
+      }
+      if (team == 16) {
+        launch_list_post<16>(C, q);
+      } else if (team == 4) {
+        launch_list_post<4>(C, q);
+      } else {
+        launch_list_post<1>(C, q);
+      }
+      C.group_end(tok);
+    }
     C.keys_valid = true;
     C.order_valid = true;
-    if (C.P.post_integrate == TG_POST_SHIFTING) {
-      e = enqueue_post(C);
-      if (e != cudaSuccess) return e;
-    }
     return step_end(C);
+  }
+
+  // The face passes' view of a stage: its positions and records, and (past
+  // the first stage) the current cells.
+  static StageArgs<D, F> list_stage_view(const ListArgs<D, F>& A) {
+    StageArgs<D, F> a = A.S;
+    for (int k = 0; k < D; ++k) a.Y.pos[k] = A.pin[k];
+    a.datrec = A.dat_in;
+    if (!A.first && a.fc.on) a.skey = A.curkey;
+    return a;
+  }
+  template<int Team>
+  void launch_list_post(Context& C, const ListPostArgs<D, F>& q) {
+    const unsigned grid = grid_for(C.n * Team, 128);
+    k_lpost_sums<D, F, K, Team><<<grid, 128, 0, C.stream>>>(q);
+    k_lpost_phi<D, F, Team><<<grid, 128, 0, C.stream>>>(q);
+    k_lpost_near<D, F, K, Team><<<grid, 128, 0, C.stream>>>(q);
+    k_lpost_shift<D, F><<<grid_for(C.n, 128), 128, 0, C.stream>>>(q);
+    k_lpost_fs<D, F, K, Team><<<grid, 128, 0, C.stream>>>(q);
+    C.launches += 5;
+  }
+  PostArgs<D, F> post_args(const Context& C) const {
+    PostArgs<D, F> p = post_;
+    p.cos2_fov = C.post_cos2_fov;
+    p.k_fs = C.post_k_fs;
+    p.shift = -C.P.cfl * 0.2;
+    return p;
   }
 
   // Lanes per target of the list passes: one where the particles alone give
@@ -598,11 +649,8 @@ class Engine final : public EngineBase {
       enqueue_gamma(C, a);
       launch_walls(C, a);
     }
-    PostArgs<D, F> p = post_;
+    PostArgs<D, F> p = post_args(C);
     p.S = a;
-    p.cos2_fov = C.post_cos2_fov;
-    p.k_fs = C.post_k_fs;
-    p.shift = -C.P.cfl * 0.2;
     const unsigned grid = grid_for(C.n, 128);
     if (C.faces.on) {
       with_face_real(C, [&](auto real) {

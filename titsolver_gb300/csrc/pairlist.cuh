@@ -63,6 +63,8 @@ struct ListArgs {
   int cap;                // entries per slot, a multiple of 4
   float margin;           // acceleration share of delta, in R
   int first, last;
+  int post;               // the last stage of a step with post-integration:
+                          // keeps the rates in Y and leaves X to that
   double w0;              // 1 - S.w_new, and both in the form's type
   R w0r, wr;
 };
@@ -976,7 +978,8 @@ __device__ __forceinline__ void list_epilogue(const ListArgs<D, F>& A, int64_t i
   // The displacement since the step's start, for the bound: dt v in the
   // first stage, so that the second starts from u_n + dt v_n and ends at
   // w dt (v_n + v) from u_n (few FP64 operations: their pipe is what the
-  // compensated form's update is bound by).
+  // compensated form's update is bound by); the third's only where
+  // post-integration follows, from the positions.
   float dis[3] = {0.f, 0.f, 0.f};
   if (S.lincomb) {
     const R wr = A.wr, w0r = A.w0r;
@@ -994,6 +997,14 @@ __device__ __forceinline__ void list_epilogue(const ListArgs<D, F>& A, int64_t i
   }
   if (!A.last) {
     float d2 = 0.f;
+    if (A.post) {
+#pragma unroll
+      for (int k = 0; k < D; ++k) {
+        dis[k] = __double2float_rn(pn[k] - S.Y.pos[k][i]);
+        S.Y.dv[k][i] = dv[k];
+      }
+      S.Y.drho[i] = drho;
+    }
 #pragma unroll
     for (int k = 0; k < D; ++k) {
       d2 = fmaf(dis[k], dis[k], d2);

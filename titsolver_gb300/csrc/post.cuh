@@ -213,6 +213,64 @@ __global__ void __launch_bounds__(128) k_post_faces(PostArgs<D, F> A) {
   }
 }
 
+// The sums of a fluid particle: the shift direction (raw N), and N, grad v
+// and grad rho renormalised by the inverse of L^T.
+template<int D, int F>
+__device__ __forceinline__ void post_store_sums(const PostArgs<D, F>& A, int64_t i, double* N,
+                                                const double* L, double* gv, double* gr,
+                                                int32_t count) {
+  double* dr = A.dr + i * D;
+#pragma unroll
+  for (int a = 0; a < D; ++a) dr[a] = N[a];
+  double LT[D * D], Li[D * D];
+#pragma unroll
+  for (int a = 0; a < D; ++a) {
+#pragma unroll
+    for (int b = 0; b < D; ++b) LT[a * D + b] = L[b * D + a];
+  }
+  if (lu_inverse<D>(LT, Li)) {
+    double tN[D], tg[D], tgv[D * D];
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+      tN[a] = 0.0;
+      tg[a] = 0.0;
+#pragma unroll
+      for (int b = 0; b < D; ++b) {
+        tN[a] += Li[a * D + b] * N[b];
+        tg[a] += Li[a * D + b] * gr[b];
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+#pragma unroll
+      for (int b = 0; b < D; ++b) {
+        double s = 0.0;
+#pragma unroll
+        for (int l = 0; l < D; ++l) s += gv[a * D + l] * Li[b * D + l];
+        tgv[a * D + b] = s;
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < D; ++a) {
+      N[a] = tN[a];
+      gr[a] = tg[a];
+    }
+#pragma unroll
+    for (int a = 0; a < D * D; ++a) gv[a] = tgv[a];
+  }
+  // normalize() with the |N|^2 >= tiny^2 guard (core/_vec/vec.hpp:663-676).
+  const double tiny2 = 6.0554544523933395e-06 * 6.0554544523933395e-06;
+  const double n2 = dot_rn(N, N, D);
+  const double sN = n2 >= tiny2 ? 1.0 / sqrt(n2) : 0.0;
+#pragma unroll
+  for (int a = 0; a < D; ++a) A.N[i * D + a] = N[a] * sN;
+#pragma unroll
+  for (int a = 0; a < D * D; ++a) A.gv[i * D * D + a] = gv[a];
+#pragma unroll
+  for (int a = 0; a < D; ++a) A.grho[i * D + a] = gr[a];
+  A.count[i] = count;
+}
+
 template<int D, int F, int K>
 __global__ void __launch_bounds__(128) k_post_sums(PostArgs<D, F> A) {
   int64_t i;
@@ -288,55 +346,7 @@ __global__ void __launch_bounds__(128) k_post_sums(PostArgs<D, F> A) {
       }
     }
   });
-  double* dr = A.dr + i * D;
-#pragma unroll
-  for (int a = 0; a < D; ++a) dr[a] = N[a];
-  double LT[D * D], Li[D * D];
-#pragma unroll
-  for (int a = 0; a < D; ++a) {
-#pragma unroll
-    for (int b = 0; b < D; ++b) LT[a * D + b] = L[b * D + a];
-  }
-  if (lu_inverse<D>(LT, Li)) {
-    double tN[D], tg[D], tgv[D * D];
-#pragma unroll
-    for (int a = 0; a < D; ++a) {
-      tN[a] = 0.0;
-      tg[a] = 0.0;
-#pragma unroll
-      for (int b = 0; b < D; ++b) {
-        tN[a] += Li[a * D + b] * N[b];
-        tg[a] += Li[a * D + b] * gr[b];
-      }
-    }
-#pragma unroll
-    for (int a = 0; a < D; ++a) {
-#pragma unroll
-      for (int b = 0; b < D; ++b) {
-        double s = 0.0;
-#pragma unroll
-        for (int l = 0; l < D; ++l) s += gv[a * D + l] * Li[b * D + l];
-        tgv[a * D + b] = s;
-      }
-    }
-#pragma unroll
-    for (int a = 0; a < D; ++a) {
-      N[a] = tN[a];
-      gr[a] = tg[a];
-    }
-#pragma unroll
-    for (int a = 0; a < D * D; ++a) gv[a] = tgv[a];
-  }
-  // normalize() with the |N|^2 >= tiny^2 guard (core/_vec/vec.hpp:663-676).
-  const double n2 = dot_rn(N, N, D);
-  const double sN = n2 >= tiny2 ? 1.0 / sqrt(n2) : 0.0;
-#pragma unroll
-  for (int a = 0; a < D; ++a) A.N[i * D + a] = N[a] * sN;
-#pragma unroll
-  for (int a = 0; a < D * D; ++a) A.gv[i * D * D + a] = gv[a];
-#pragma unroll
-  for (int a = 0; a < D; ++a) A.grho[i * D + a] = gr[a];
-  A.count[i] = count;
+  post_store_sums<D, F>(A, i, N, L, gv, gr, count);
 }
 
 template<int D, int F>
@@ -430,29 +440,11 @@ __global__ void __launch_bounds__(128) k_post_near(PostArgs<D, F> A) {
   A.phi2[i] = out;
 }
 
+// Position, velocity and density of a far particle after its shift.
 template<int D, int F>
-__global__ void __launch_bounds__(128) k_post_shift(PostArgs<D, F> A) {
-  using R = typename StageArgs<D, F>::R;
-  int64_t i;
-  uint32_t id;
-  const TankDev* Tp;
-  int c[3] = {0, 0, 0};
-  if (!post_target(A, i, id, Tp, c)) return;
-  if (id & kWallBit) {
-    commit_wall(A.S, i, id);
-    return;
-  }
-  const TankDev& T = *Tp;
-  const StateBuf<R>& Y = A.S.Y;
-  const StateBuf<R>& X = A.S.X;
-  double p[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-  for (int k = 0; k < D; ++k) {
-    p[k] = Y.pos[k][i];
-    v[k] = static_cast<double>(Y.vel[k][i]);
-  }
-  double rho = static_cast<double>(Y.rho[i]);
-  if constexpr (F == TG_FP32C) rho += T.rho0;
+__device__ __forceinline__ void post_apply_shift(const PostArgs<D, F>& A, int64_t i,
+                                                 const TankDev& T, double* p, double* v,
+                                                 double& rho) {
   if (bits_eq(A.phi2[i], kPhiMax)) {
     const double sc = A.shift * (T.h * T.h);
     double dr[D];
@@ -471,12 +463,21 @@ __global__ void __launch_bounds__(128) k_post_shift(PostArgs<D, F> A) {
     }
     rho += dot_rn(A.grho + i * D, dr, D);
   }
-  A.rho_raw[i] = rho;
-  // Home state with the key (and FP32 offset) of the new position.
+}
+
+// Home state of a fluid particle with the key (and FP32 offset) of its new
+// position; key: its key in this sort.
+template<int D, int F>
+__device__ __forceinline__ void post_commit(const StageArgs<D, F>& S, int64_t i, uint32_t id,
+                                            uint32_t key, const TankDev& T, const double* p,
+                                            const double* v, double rho,
+                                            const typename StageArgs<D, F>::R* dv,
+                                            typename StageArgs<D, F>::R drho) {
+  const auto& X = S.X;
   int cn[3] = {0, 0, 0};
   bool outside = false;
   cell_of<D>(T, p, cn, outside);
-  if (outside) atomicOr(A.S.err, static_cast<uint32_t>(TG_DEV_OUTSIDE_GRID));
+  if (outside) atomicOr(S.err, static_cast<uint32_t>(TG_DEV_OUTSIDE_GRID));
   bool finite = true;
 #pragma unroll
   for (int k = 0; k < D; ++k) {
@@ -487,7 +488,7 @@ __global__ void __launch_bounds__(128) k_post_shift(PostArgs<D, F> A) {
       X.vel[k][i] = __double2float_rn(v[k]);
       X.off[k][i] = __double2float_rn(p[k] - fma(static_cast<double>(cn[k]), T.cs, T.lo[k]));
     }
-    X.dv[k][i] = Y.dv[k][i];
+    X.dv[k][i] = dv[k];
     finite = finite && finite_bits(p[k]) && finite_bits(v[k]);
   }
   if constexpr (F == TG_FP64) {
@@ -495,12 +496,63 @@ __global__ void __launch_bounds__(128) k_post_shift(PostArgs<D, F> A) {
   } else {
     X.rho[i] = __double2float_rn(rho - T.rho0);
   }
-  X.drho[i] = Y.drho[i];
+  X.drho[i] = drho;
   X.id[i] = id;
-  X.pkey[i] = A.S.skey[i];  // read before the key write: the buffers may alias
+  X.pkey[i] = key;  // read before the key write: the buffers may alias
   X.key[i] = key_of(flat_cell<D>(T, cn), false);
   if (!(finite && finite_bits(rho))) {
-    atomicOr(A.S.err, static_cast<uint32_t>(TG_DEV_NONFINITE_STATE));
+    atomicOr(S.err, static_cast<uint32_t>(TG_DEV_NONFINITE_STATE));
+  }
+}
+
+template<int D, int F>
+__global__ void __launch_bounds__(128) k_post_shift(PostArgs<D, F> A) {
+  using R = typename StageArgs<D, F>::R;
+  int64_t i;
+  uint32_t id;
+  const TankDev* Tp;
+  int c[3] = {0, 0, 0};
+  if (!post_target(A, i, id, Tp, c)) return;
+  if (id & kWallBit) {
+    commit_wall(A.S, i, id);
+    return;
+  }
+  const TankDev& T = *Tp;
+  const StateBuf<R>& Y = A.S.Y;
+  double p[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    p[k] = Y.pos[k][i];
+    v[k] = static_cast<double>(Y.vel[k][i]);
+  }
+  double rho = static_cast<double>(Y.rho[i]);
+  if constexpr (F == TG_FP32C) rho += T.rho0;
+  post_apply_shift<D, F>(A, i, T, p, v, rho);
+  A.rho_raw[i] = rho;
+  R dv[3] = {R(0), R(0), R(0)};
+#pragma unroll
+  for (int k = 0; k < D; ++k) dv[k] = Y.dv[k][i];
+  post_commit<D, F>(A.S, i, id, A.S.skey[i], T, p, v, rho, dv, Y.drho[i]);
+}
+
+// The corrected density of a near-surface particle from its Shepard sum
+// alpha and its summation density.
+template<int D, int F>
+__device__ __forceinline__ void post_commit_density(const PostArgs<D, F>& A,
+                                                    const StageArgs<D, F>& S, int64_t i,
+                                                    const TankDev& T, double alpha,
+                                                    double rho_t) {
+  const double gam = S.fc.on ? S.fc.gamma[i] : 1.0;
+  const double ratio = fmin(1.0, alpha / gam);
+  if (ratio > 0.99) return;
+  const double beta = exp(-A.k_fs * ((ratio - 1.0) * (ratio - 1.0)));
+  const double corr = beta * gam + (1.0 - beta) * alpha;
+  if (fabs(corr) <= 6.0554544523933395e-06) return;
+  const double rho = rho_t / corr;
+  if constexpr (F == TG_FP64) {
+    S.X.rho[i] = rho;
+  } else {
+    S.X.rho[i] = __double2float_rn(rho - T.rho0);
   }
 }
 
@@ -536,18 +588,7 @@ __global__ void __launch_bounds__(128) k_post_fs(PostArgs<D, F> A) {
       rho_t += T.m * W;
     }
   });
-  const double gam = A.S.fc.on ? A.S.fc.gamma[i] : 1.0;
-  const double ratio = fmin(1.0, alpha / gam);
-  if (ratio > 0.99) return;
-  const double beta = exp(-A.k_fs * ((ratio - 1.0) * (ratio - 1.0)));
-  const double corr = beta * gam + (1.0 - beta) * alpha;
-  if (fabs(corr) <= 6.0554544523933395e-06) return;
-  const double rho = rho_t / corr;
-  if constexpr (F == TG_FP64) {
-    A.S.X.rho[i] = rho;
-  } else {
-    A.S.X.rho[i] = __double2float_rn(rho - T.rho0);
-  }
+  post_commit_density<D, F>(A, A.S, i, T, alpha, rho_t);
 }
 
 }  // namespace tg
