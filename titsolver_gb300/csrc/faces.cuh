@@ -80,7 +80,7 @@ struct FaceArgs {
   int on;
 };
 
-// Block size of the warp-per-face-particle passes (their shared queues are
+// Block size of the passes over the face particles (their shared queues are
 // sized by it).
 constexpr int kFaceBlock = 128;
 
@@ -843,14 +843,42 @@ __device__ __forceinline__ unsigned face_skip_edges(const FaceArgs& fc, uint32_t
   return skip;
 }
 
+// Lanes per face particle.  3D: a warp (its triangles' edges are shared out
+// over one).  2D: a particle has about nine segments within reach, so a warp
+// takes two particles (pool of 12,800 fluid particles, four steps: 4490 us
+// with 16 lanes, 5577 with 32, 5224 with 8, 5512 with 4: the fewer lanes, the
+// longer each particle's chain of FP64 operations).
+template<int D>
+constexpr int face_group() {
+  return D == 2 ? 16 : 32;
+}
+// The group's lanes in its warp, and this lane's place in the group.
+template<int D>
+__device__ __forceinline__ unsigned face_mask() {
+  constexpr int G = face_group<D>();
+  if constexpr (G == 32) return 0xffffffffu;
+  else return ((1u << G) - 1u) << (threadIdx.x & 31u & ~static_cast<unsigned>(G - 1));
+}
+template<int D>
+__device__ __forceinline__ int face_lane() {
+  return static_cast<int>(threadIdx.x) & (face_group<D>() - 1);
+}
+// Sum over the lanes of a group (all active), butterfly order.
+template<int D>
+__device__ __forceinline__ double face_sum(double v) {
+#pragma unroll
+  for (int o = face_group<D>() / 2; o > 0; o >>= 1) v += __shfl_xor_sync(face_mask<D>(), v, o);
+  return v;
+}
+
 // Faces within the support radius of x (the particle's cell list holds
-// every face within reach of the cell), shared by the lanes of a warp: the
-// lanes test 32 list entries at a time and queue the faces that pass in a
-// per-warp shared buffer, and every full batch of 32 queued faces is
+// every face within reach of the cell), shared by the lanes of a group: the
+// lanes test one list entry each at a time and queue the faces that pass in
+// a shared buffer of the group, and every full batch of queued faces is
 // integrated with one face per lane (the rest at the end, with the idle
-// lanes inactive), so the costly integrals run on full warps.  fn(active,
-// f, coords) is called by all 32 lanes together.  Blocks of kFaceBlock
-// threads.
+// lanes inactive), so the costly integrals run on full groups.  fn(active,
+// f, coords) is called by all lanes of the group together.  Blocks of
+// kFaceBlock threads.
 
 template<int D, class Fn>
 __device__ __forceinline__ void for_adjacent_faces(const FaceArgs& fc,
@@ -858,11 +886,13 @@ __device__ __forceinline__ void for_adjacent_faces(const FaceArgs& fc,
                                                    const double* x,
                                                    double radius, int lane,
                                                    Fn&& fn) {
-  __shared__ uint32_t queue[kFaceBlock / 32][64];
-  uint32_t* q = queue[threadIdx.x >> 5];
+  constexpr int G = face_group<D>();
+  __shared__ uint32_t queue[kFaceBlock / G][2 * G];
+  uint32_t* q = queue[threadIdx.x / G];
+  const unsigned group = face_mask<D>(), below = group & ((1u << (threadIdx.x & 31u)) - 1u);
   const uint32_t s = fc.cell_start[gcell], e = fc.cell_start[gcell + 1];
   int pending = 0;
-  for (uint32_t base = s; base < e; base += 32) {
+  for (uint32_t base = s; base < e; base += G) {
     const uint32_t i = base + static_cast<uint32_t>(lane);
     bool in = false;
     uint32_t f = 0;
@@ -872,14 +902,14 @@ __device__ __forceinline__ void for_adjacent_faces(const FaceArgs& fc,
       if constexpr (D == 2) in = segment_in_sphere(g, x, radius);
       else in = triangle_in_sphere(g, x, radius);
     }
-    const unsigned mask = __ballot_sync(0xffffffffu, in);
-    if (in) q[pending + __popc(mask & ((1u << lane) - 1u))] = f;
+    const unsigned mask = __ballot_sync(group, in) & group;
+    if (in) q[pending + __popc(mask & below)] = f;
     pending += __popc(mask);
-    __syncwarp();
-    if (pending >= 32) {
-      pending -= 32;
+    __syncwarp(group);
+    if (pending >= G) {
+      pending -= G;
       const uint32_t g = q[pending + lane];
-      __syncwarp();
+      __syncwarp(group);
       fn(true, g, fc.coords + D * D * static_cast<size_t>(g));
     }
   }
@@ -888,25 +918,28 @@ __device__ __forceinline__ void for_adjacent_faces(const FaceArgs& fc,
     const uint32_t g = q[active ? lane : 0];
     fn(active, g, fc.coords + D * D * static_cast<size_t>(g));
   }
-  __syncwarp();
+  __syncwarp(group);
 }
 
-// Capacity of the per-warp list of a face particle's in-range faces
+// Capacity of the list of a face particle's in-range faces
 // (collect_adjacent_faces); a particle with more takes the list-free path.
-constexpr int kFaceListCap = 256;
+template<int D>
+constexpr int kFaceListCap = D == 2 ? 64 : 256;
 
 // The faces of the particle's cell list within the support radius of x
-// (the for_adjacent_faces predicate), ascending, into the warp's list; all
+// (the for_adjacent_faces predicate), ascending, into the group's list; all
 // lanes call and get the count.  A count above cap means the list holds
 // only the first cap faces.
 template<int D>
 __device__ __forceinline__ int collect_adjacent_faces(const FaceArgs& fc, uint32_t gcell,
                                                       const double* x, double radius,
                                                       int lane, uint32_t* list, int cap) {
-  __syncwarp();  // the previous particle's readers are done with the list
+  constexpr int G = face_group<D>();
+  const unsigned group = face_mask<D>(), below = group & ((1u << (threadIdx.x & 31u)) - 1u);
+  __syncwarp(group);  // the previous particle's readers are done with the list
   const uint32_t s = fc.cell_start[gcell], e = fc.cell_start[gcell + 1];
   int count = 0;
-  for (uint32_t base = s; base < e; base += 32) {
+  for (uint32_t base = s; base < e; base += G) {
     const uint32_t i = base + static_cast<uint32_t>(lane);
     bool in = false;
     uint32_t f = 0;
@@ -916,12 +949,12 @@ __device__ __forceinline__ int collect_adjacent_faces(const FaceArgs& fc, uint32
       if constexpr (D == 2) in = segment_in_sphere(g, x, radius);
       else in = triangle_in_sphere(g, x, radius);
     }
-    const unsigned mask = __ballot_sync(0xffffffffu, in);
-    const int slot = count + __popc(mask & ((1u << lane) - 1u));
+    const unsigned mask = __ballot_sync(group, in) & group;
+    const int slot = count + __popc(mask & below);
     if (in && slot < cap) list[slot] = f;
     count += __popc(mask);
   }
-  __syncwarp();
+  __syncwarp(group);
   return count;
 }
 

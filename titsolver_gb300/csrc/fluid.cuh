@@ -1325,15 +1325,16 @@ __device__ __forceinline__ double face_avg(const double* x) {
 }
 
 // Face terms of continuity and momentum (fluid_equations.hpp:241-247,
-// 278-291) of the face particles, one warp per particle with the lanes
+// 278-291) of the face particles, one group per particle with the lanes
 // splitting its faces; k_gamma_init zeroed the other particles' terms.
 template<int D, int K, int F, class FT>
 __global__ void __launch_bounds__(128) k_face_terms(StageArgs<D, F> A) {
   const FaceArgs& fc = A.fc;
-  const int lane = threadIdx.x & 31;
-  const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
+  constexpr int G = face_group<D>();
+  const int lane = face_lane<D>();
+  const uint32_t groups = gridDim.x * (blockDim.x / G);
   const uint32_t count = *fc.face_count;
-  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < count; w += nwarps) {
+  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) / G; w < count; w += groups) {
     const uint32_t i = fc.face_list[w];
     if (A.Y.id[i] & kWallBit) continue;
     const uint32_t key = A.skey[i];
@@ -1388,9 +1389,9 @@ __global__ void __launch_bounds__(128) k_face_terms(StageArgs<D, F> A) {
 #pragma unroll
       for (int k = 0; k < D; ++k) dv[k] += (P_as * gg[k] - Pi_s * t_as[k] * ng) / gam;
     });
-    drho = warp_sum(drho);
+    drho = face_sum<D>(drho);
 #pragma unroll
-    for (int k = 0; k < D; ++k) dv[k] = warp_sum(dv[k]);
+    for (int k = 0; k < D; ++k) dv[k] = face_sum<D>(dv[k]);
     if (lane == 0) {
       fc.face_drho[i] = drho;
 #pragma unroll
@@ -2133,7 +2134,7 @@ __global__ void __launch_bounds__(128) k_sumdens(CloudArgs<D> A) {
 // records the cell-order slot of each fixed particle (for the face terms'
 // vertex lookups) and lists the face particles, those whose cell lists
 // faces; the others have grad gamma = 0, gamma = the containment answer,
-// and zero face terms.  k_gamma_faces, one warp per face particle with the
+// and zero face terms.  k_gamma_faces, one group per face particle with the
 // lanes splitting its faces: grad gamma = the sum of kernel fluxes, then
 // gamma = contains - the sum of antigradient fluxes at r + (2 contains - 1)
 // n h^2.  A fixed particle's gamma is never read (its grad gamma gives the
@@ -2177,13 +2178,14 @@ __global__ void __launch_bounds__(128) k_gamma_init(StageArgs<D, F> A) {
 
 template<int D, int K, int F, class FT>
 __global__ void __launch_bounds__(128) k_gamma_faces(StageArgs<D, F> A) {
-  __shared__ uint32_t flist_all[kFaceBlock / 32][kFaceListCap];
+  __shared__ uint32_t flist_all[kFaceBlock / face_group<D>()][kFaceListCap<D>];
   const FaceArgs& fc = A.fc;
-  const int lane = threadIdx.x & 31;
-  uint32_t* flist = flist_all[threadIdx.x >> 5];
-  const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
+  constexpr int G = face_group<D>();
+  const int lane = face_lane<D>();
+  uint32_t* flist = flist_all[threadIdx.x / G];
+  const uint32_t groups = gridDim.x * (blockDim.x / G);
   const uint32_t count = *fc.face_count;
-  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < count; w += nwarps) {
+  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) / G; w < count; w += groups) {
     const uint32_t i = fc.face_list[w];
     const bool wall = (A.Y.id[i] & kWallBit) != 0;
     const uint32_t key = A.skey[i];
@@ -2201,10 +2203,10 @@ __global__ void __launch_bounds__(128) k_gamma_faces(StageArgs<D, F> A) {
     // sweep at xs keeps the adjacency of x); the skip masks come from the
     // same list.  Past the list's capacity both sweeps test the cell list
     // again, as for_adjacent_faces does.
-    const int nf = collect_adjacent_faces<D>(fc, gcell, x, radius, lane, flist, kFaceListCap);
+    const int nf = collect_adjacent_faces<D>(fc, gcell, x, radius, lane, flist, kFaceListCap<D>);
     auto sweep = [&](auto&& fn) {
-      if (nf <= kFaceListCap) {
-        for (int base = 0; base < nf; base += 32) {
+      if (nf <= kFaceListCap<D>) {
+        for (int base = 0; base < nf; base += G) {
           const bool active = base + lane < nf;
           const uint32_t fi = flist[active ? base + lane : base];
           const unsigned skip = active ? face_skip_edges_listed<D>(fc, fi, flist, nf) : 0u;
@@ -2227,7 +2229,7 @@ __global__ void __launch_bounds__(128) k_gamma_faces(StageArgs<D, F> A) {
       for (int k = 0; k < D; ++k) g[k] += fl[k];
     });
 #pragma unroll
-    for (int k = 0; k < D; ++k) g[k] = warp_sum(g[k]);
+    for (int k = 0; k < D; ++k) g[k] = face_sum<D>(g[k]);
     if (lane == 0) {
 #pragma unroll
       for (int k = 0; k < D; ++k) fc.ggam[D * i + k] = g[k];
@@ -2253,7 +2255,7 @@ __global__ void __launch_bounds__(128) k_gamma_faces(StageArgs<D, F> A) {
             face_antigrad_flux_d<K, D, FT>(active, f, face_axes<D>(fc, fi), xs, T.h, wd, skip);
         if (active) ag += a;
       });
-      ga -= warp_sum(ag);
+      ga -= face_sum<D>(ag);
     }
     if (lane == 0) fc.gamma[i] = ga;
   }

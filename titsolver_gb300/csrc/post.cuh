@@ -147,17 +147,18 @@ __device__ __forceinline__ bool post_target(const PostArgs<D, F>& A, int64_t& i,
 
 // Face terms of the shifting sums of the fluid face particles (N, L,
 // grad v, grad rho; fluid_equations.hpp:340-349), divided by gamma_a, one
-// warp per particle with the lanes splitting its faces; k_post_sums starts
+// group per particle with the lanes splitting its faces; k_post_sums starts
 // its pair sums from them (zero for particles whose cell lists no faces).
 // A pass of its own keeps the face integrals' registers out of the pair
 // loop.
 template<int D, int F, int K, class FT>
 __global__ void __launch_bounds__(128) k_post_faces(PostArgs<D, F> A) {
   const FaceArgs& fc = A.S.fc;
-  const int lane = threadIdx.x & 31;
-  const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
+  constexpr int G = face_group<D>();
+  const int lane = face_lane<D>();
+  const uint32_t groups = gridDim.x * (blockDim.x / G);
   const uint32_t count = *fc.face_count;
-  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < count; w += nwarps) {
+  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) / G; w < count; w += groups) {
     const uint32_t i = fc.face_list[w];
     if (A.S.Y.id[i] & kWallBit) continue;
     const uint32_t key = A.S.skey[i];
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(128) k_post_faces(PostArgs<D, F> A) {
     double* out = fc.post_face + kPostFaceSums<D> * static_cast<size_t>(i);
 #pragma unroll
     for (int k = 0; k < kPostFaceSums<D>; ++k) {
-      const double v = warp_sum(sums[k]);
+      const double v = face_sum<D>(sums[k]);
       if (lane == 0) out[k] = v;
     }
   }
