@@ -4,6 +4,7 @@
 
 #include <memory>
 
+#include "density.cuh"
 #include "engine.cuh"
 #include "fluid.cuh"
 #include "pairlist.cuh"
@@ -298,26 +299,30 @@ class Engine final : public EngineBase {
     cudaError_t e = enqueue_sort(C);
     if (e != cudaSuccess) return e;
     const bool f32 = pos_precision == TG_POS_FP32;
+    // The staging buffers hold the local coordinates or the hashes.
+    float* l = reinterpret_cast<float*>(C.d_stage);
+    auto* hash = reinterpret_cast<uint64_t*>(C.d_stage2);
+    const CloudArgs<D> ca{C.d_cloud_rec, {l, l + C.n, l + 2 * C.n}, hash, Y_.id, C.sorted_keys,
+                          C.cell_start,  C.d_tanks, C.d_tank_off, C.ntanks, C.n, C.k, rho,
+                          counts,        hashes,    C.d_id_base};
     int tok = C.group_begin(kGroupReorder);
+    const unsigned g = grid_for(C.n, 256);
     if (f32) {
-      k_cloud_records<D, true><<<grid_for(C.n, 256), 256, 0, C.stream>>>(
-          X_.pos[0], X_.pos[1], X_.pos[2], X_.id, C.perm, C.d_cloud_rec,
-          Y_.id, C.n);
+      k_cloud_records<D, true><<<g, 256, 0, C.stream>>>(
+          X_.pos[0], X_.pos[1], X_.pos[2], X_.id, C.perm, ca, C.d_cloud_rec, Y_.id, l, l + C.n,
+          l + 2 * C.n, hash);
     } else {
-      k_cloud_records<D, false><<<grid_for(C.n, 256), 256, 0, C.stream>>>(
-          X_.pos[0], X_.pos[1], X_.pos[2], X_.id, C.perm, C.d_cloud_rec,
-          Y_.id, C.n);
+      k_cloud_records<D, false><<<g, 256, 0, C.stream>>>(
+          X_.pos[0], X_.pos[1], X_.pos[2], X_.id, C.perm, ca, C.d_cloud_rec, Y_.id, l, l + C.n,
+          l + 2 * C.n, hash);
     }
     C.launches += 1;
     C.group_end(tok);
-    CloudArgs<D> ca{C.d_cloud_rec, Y_.id, C.sorted_keys, C.cell_start,
-                    C.d_tanks,     C.d_tank_off, C.ntanks, C.n,
-                    C.k,           rho,   counts, hashes,  C.d_id_base};
     tok = C.group_begin(kGroupForces);
     if (f32) {
-      k_sumdens<D, K, true><<<grid_for(C.n, 128), 128, 0, C.stream>>>(ca);
+      k_density32<D, K><<<grid_for(C.n, kDensityBlock), kDensityBlock, 0, C.stream>>>(ca);
     } else {
-      k_sumdens<D, K, false><<<grid_for(C.n, 128), 128, 0, C.stream>>>(ca);
+      k_density64<D, K><<<grid_for(C.n * 32, kDensityBlock), kDensityBlock, 0, C.stream>>>(ca);
     }
     C.launches += 1;
     C.group_end(tok);

@@ -331,11 +331,12 @@ __device__ __forceinline__ void cell_offset(const TankDev& T, const int* c,
 }
 
 // Clipped x-range of one row: [x0, x1] within [xlo, xhi]; false when the
-// row holds no reachable cell.
+// row holds no reachable cell.  cull2: the cull radius squared.
 template<int D>
 __device__ __forceinline__ bool clip_row(const TankDev& T, const int* c,
                                          const float* o, int y, int z,
-                                         int xlo, int xhi, int& x0, int& x1) {
+                                         int xlo, int xhi, int& x0, int& x1,
+                                         float cull2) {
   x0 = xlo;
   x1 = xhi;
   if (o == nullptr) return true;
@@ -345,7 +346,7 @@ __device__ __forceinline__ bool clip_row(const TankDev& T, const int* c,
   if constexpr (D == 3) {
     gz = (z == 0 || z == T.nc[2] - 1) ? 0.f : cell_gap(z - c[2], o[2], cs);
   }
-  const float rem = T.cull_r2_f - gy * gy - gz * gz;
+  const float rem = cull2 - gy * gy - gz * gz;
   if (rem < 0.f) return false;
   if (xlo == 0 || xhi == T.nc[0] - 1) return true;
   const float w = sqrtf(rem);
@@ -373,7 +374,7 @@ __device__ __forceinline__ void for_cells(const TankDev& T, const int* c,
   for (int z = zlo; z <= zhi; ++z) {
     for (int y = ylo; y <= yhi; ++y) {
       int x0, x1;
-      if (!clip_row<D>(T, c, o, y, z, xlo, xhi, x0, x1)) continue;
+      if (!clip_row<D>(T, c, o, y, z, xlo, xhi, x0, x1, T.cull_r2_f)) continue;
       const uint32_t row =
           T.cell_off + (static_cast<uint32_t>(z) * ny + y) * nx;
       if constexpr (!PerCell) {
@@ -445,6 +446,39 @@ __device__ __forceinline__ void for_cells_team(
   }
 }
 
+// The rows of the (2k+1)^D cell block around c, each shared by the Team
+// lanes of a target's team: every lane looks up the record range of one row
+// of a batch (clipped as in for_cells, to the cull radius squared cull2),
+// and fn(s, e) is called by all lanes for each of them in turn.
+template<int D, int Team, class Fn>
+__device__ __forceinline__ void for_shared_rows(const TankDev& T, const int* c, int k,
+                                                const uint32_t* __restrict__ cstart, int lane,
+                                                unsigned mask, const float* o, float cull2,
+                                                Fn&& fn) {
+  const int nx = T.nc[0], ny = T.nc[1];
+  const int xlo = max(c[0] - k, 0), xhi = min(c[0] + k, nx - 1);
+  const int span = 2 * k + 1, rows = D == 3 ? span * span : span;
+  for (int t0 = 0; t0 < rows; t0 += Team) {
+    const int t = t0 + lane;
+    const int y = c[1] - k + t % span;
+    const int z = D == 3 ? c[2] - k + t / span : 0;
+    uint32_t s = 0, e = 0;
+    if (t < rows && y >= 0 && y < ny && z >= 0 && z < T.nc[2]) {
+      int x0, x1;
+      if (clip_row<D>(T, c, o, y, z, xlo, xhi, x0, x1, cull2)) {
+        const uint32_t row = T.cell_off + (static_cast<uint32_t>(z) * ny + y) * nx;
+        s = __ldg(cstart + 2 * (row + x0));
+        e = __ldg(cstart + 2 * (row + x1 + 1));
+      }
+    }
+#pragma unroll 1
+    for (unsigned full = __ballot_sync(mask, s < e) & mask; full != 0u; full &= full - 1u) {
+      const int src = __ffs(full) - 1;
+      fn(__shfl_sync(mask, s, src), __shfl_sync(mask, e, src));
+    }
+  }
+}
+
 // Rows of the (2k+1)^D cell block around c (3D), dealt out to the lanes of
 // a team: lane l visits rows l, l + team, ...; each visit gets the row's
 // whole record range (fluid and walls, clipped as in for_cells) and its
@@ -465,7 +499,7 @@ __device__ __forceinline__ void for_rows_team(
     const int y = ylo + t % wy;
     const int z = zlo + t / wy;
     int x0, x1;
-    if (!clip_row<D>(T, c, o, y, z, xlo, xhi, x0, x1)) continue;
+    if (!clip_row<D>(T, c, o, y, z, xlo, xhi, x0, x1, T.cull_r2_f)) continue;
     const uint32_t row = T.cell_off + (static_cast<uint32_t>(z) * ny + y) * nx;
     fn(__ldg(cstart + 2 * (row + x0)), __ldg(cstart + 2 * (row + x1 + 1)), 0,
        y - c[1], D == 3 ? z - c[2] : 0);
@@ -2037,98 +2071,6 @@ __global__ void __launch_bounds__(128)
 }
 
 // ---------------------------------------------------------------------------
-// Summation density over a point cloud (fluid_equations.hpp:498-502 form,
-// self included): rho_a = sum_b m W_ab, with neighbour counts and hashes.
-// FP64 positions: FP64 predicate and sum.  FP32 positions: the positions are
-// rounded to float once; predicate and kernel in FP32, compensated sum.
-template<int D>
-struct CloudArgs {
-  const void* pos;  // Pos64_* or Pos32_* absolute positions, cell order
-  const uint32_t* id;
-  const uint32_t* skey;  // sorted keys
-  const uint32_t* cell_start;
-  const TankDev* tanks;
-  const uint32_t* tank_off;
-  int ntanks;
-  int64_t n;
-  int k;
-  double* rho;       // by upload id
-  int32_t* counts;   // by upload id
-  uint64_t* hashes;  // by upload id
-  const uint32_t* id_base;
-};
-
-template<int D, int K, bool F32>
-__global__ void __launch_bounds__(128) k_sumdens(CloudArgs<D> A) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= A.n) return;
-  const uint32_t id = A.id[i] & kIdMask;
-  const uint32_t key = A.skey[i];
-  const uint32_t tk = tank_of_key(key, A.tank_off, A.ntanks);
-  const TankDev& T = A.tanks[tk];
-  const uint32_t base = A.id_base[tk];
-  int c[3] = {0, 0, 0};
-  cell_from_key<D>(T, key, c);
-  int32_t cnt = 0;
-  uint64_t hs = 0;
-  double rho;
-  if constexpr (!F32) {
-    using P = std::conditional_t<D == 2, Pos64_2, Pos64_3>;
-    const P* pr = static_cast<const P*>(A.pos);
-    double pa[3] = {0.0, 0.0, 0.0};
-    load_pos(pr, static_cast<uint32_t>(i), pa);
-    const double R2 = T.radius2, hinv = T.hinv, wm = T.w * T.m;
-    double acc = 0.0;
-    // Cell clipping where the grid carries its FP32 geometry (not in the
-    // allocation-free pass, whose grid leaves it unset).
-    float oc[3] = {0.f, 0.f, 0.f};
-    cell_offset<D>(T, c, pa, oc);
-    const float* clip = T.cull_r2_f > 0.f ? oc : nullptr;
-    for_cells<D, false>(T, c, A.k, A.cell_start,
-                        [&](uint32_t s, uint32_t en, int, int, int) {
-      for (uint32_t j = s; j < en; ++j) {
-        double pb[3], d[3];
-        load_pos(pr, j, pb);
-        const double s2 = dist2_exact<D>(pa, pb, d);
-        if (s2 > R2) continue;
-        acc += wm * KernelPoly<K>::value(sqrt(s2) * hinv);
-        ++cnt;
-        hs += splitmix64(static_cast<uint64_t>((A.id[j] & kIdMask) - base) + 1u);
-      }
-    }, clip);
-    rho = acc;
-  } else {
-    using P = std::conditional_t<D == 2, Pos32_2, Pos32_3>;
-    const P* pr = static_cast<const P*>(A.pos);
-    float pa[3] = {0.f, 0.f, 0.f};
-    load_pos(pr, static_cast<uint32_t>(i), pa);
-    const float R2 = T.radius2_f, hinv = T.hinv_f;
-    const float wm = T.w_f * T.m_f;
-    Kahan acc;
-    double pd[3] = {pa[0], pa[1], pa[2]};
-    float oc[3] = {0.f, 0.f, 0.f};
-    cell_offset<D>(T, c, pd, oc);
-    const float* clip = T.cull_r2_f > 0.f ? oc : nullptr;
-    for_cells<D, false>(T, c, A.k, A.cell_start,
-                        [&](uint32_t s, uint32_t en, int, int, int) {
-      for (uint32_t j = s; j < en; ++j) {
-        float pb[3], d[3];
-        load_pos(pr, j, pb);
-        const float s2 = dist2_exact<D>(pa, pb, d);
-        if (s2 > R2) continue;
-        acc.add(wm * KernelPoly<K>::value(sqrtf(s2) * hinv));
-        ++cnt;
-        hs += splitmix64(static_cast<uint64_t>((A.id[j] & kIdMask) - base) + 1u);
-      }
-    }, clip);
-    rho = static_cast<double>(acc.value());
-  }
-  if (A.rho != nullptr) A.rho[id] = rho;
-  if (A.counts != nullptr) A.counts[id] = cnt;
-  if (A.hashes != nullptr) A.hashes[id] = hs;
-}
-
-// ---------------------------------------------------------------------------
 // gamma and grad gamma of every particle (FluidEquations::compute_gamma,
 // fluid_equations.hpp:166-193) in two passes.  k_gamma_init, per particle:
 // records the cell-order slot of each fixed particle (for the face terms'
@@ -2408,36 +2350,6 @@ static __global__ void k_step_end(double* dt, double* dt_last, double* time, uns
     dt_last[t] = d;
   }
   dt[t] = __longlong_as_double(0x7ff0000000000000ll);
-}
-
-// Cloud records for the summation density: absolute positions in cell order
-// (FP64, or rounded once to FP32) and ids.
-template<int D, bool F32>
-__global__ void __launch_bounds__(256)
-    k_cloud_records(const double* __restrict__ px,
-                    const double* __restrict__ py,
-                    const double* __restrict__ pz,
-                    const uint32_t* __restrict__ id_in,
-                    const uint32_t* __restrict__ perm, void* rec,
-                    uint32_t* __restrict__ id_out, int64_t n) {
-  const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const uint32_t s = perm[j];
-  const double x = px[s], y = py[s], z = D == 3 ? pz[s] : 0.0;
-  if constexpr (F32) {
-    if constexpr (D == 2) {
-      static_cast<Pos32_2*>(rec)[j] = Pos32_2{float(x), float(y)};
-    } else {
-      static_cast<Pos32_3*>(rec)[j] = Pos32_3{float(x), float(y), float(z), 0.f};
-    }
-  } else {
-    if constexpr (D == 2) {
-      static_cast<Pos64_2*>(rec)[j] = Pos64_2{x, y};
-    } else {
-      static_cast<Pos64_3*>(rec)[j] = Pos64_3{x, y, z, 0.0};
-    }
-  }
-  id_out[j] = id_in[s];
 }
 
 }  // namespace tg

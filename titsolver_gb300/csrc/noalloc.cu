@@ -17,7 +17,7 @@
 #include <cstdint>
 #include <mutex>
 
-#include "fluid.cuh"
+#include "density.cuh"
 #include "sort.cuh"
 
 namespace tg {
@@ -71,18 +71,30 @@ cudaError_t scratch_address(unsigned char** out) {
   return cudaSuccess;
 }
 
-// Bounding box and cell grid of the cloud, computed on the device: cells of
-// at least the support radius (so neighbours lie within one cell), enlarged
-// when needed so the grid has at most kMaxCells cells.
+// Bounding box of the cloud: kBoxBlocks partial boxes (lo and hi per axis),
+// which k_na_grid folds; one block over all points took 130 us at 60,000.
+constexpr int kBoxBlocks = 64;
+
+template<int D>
+__device__ __forceinline__ void fold_box(double* lo, double* hi) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      lo[k] = fmin(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
+      hi[k] = fmax(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
+    }
+  }
+}
+
 template<int D>
 __global__ void __launch_bounds__(256)
-    k_na_grid(const double* __restrict__ r, int64_t n, double h, double m,
-              double unit_radius, double weight, TankDev* T,
-              uint32_t* id_base) {
-  __shared__ double s_lo[256][3], s_hi[256][3];
+    k_na_box(const double* __restrict__ r, int64_t n, double* __restrict__ boxes) {
+  __shared__ double s_lo[8][3], s_hi[8][3];
   double lo[3] = {INFINITY, INFINITY, INFINITY};
   double hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
+       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
 #pragma unroll
     for (int k = 0; k < D; ++k) {
       const double x = r[i * D + k];
@@ -90,28 +102,52 @@ __global__ void __launch_bounds__(256)
       hi[k] = fmax(hi[k], x);
     }
   }
+  fold_box<D>(lo, hi);
+  const int warp = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    s_lo[threadIdx.x][k] = lo[k];
-    s_hi[threadIdx.x][k] = hi[k];
+    for (int k = 0; k < D; ++k) {
+      s_lo[warp][k] = lo[k];
+      s_hi[warp][k] = hi[k];
+    }
   }
   __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        s_lo[threadIdx.x][k] = fmin(s_lo[threadIdx.x][k], s_lo[threadIdx.x + s][k]);
-        s_hi[threadIdx.x][k] = fmax(s_hi[threadIdx.x][k], s_hi[threadIdx.x + s][k]);
-      }
+  if (threadIdx.x < D) {
+    const int k = threadIdx.x;
+    double a = s_lo[0][k], b = s_hi[0][k];
+    for (int w = 1; w < 8; ++w) {
+      a = fmin(a, s_lo[w][k]);
+      b = fmax(b, s_hi[w][k]);
     }
-    __syncthreads();
+    boxes[(2 * blockIdx.x) * 3 + k] = a;
+    boxes[(2 * blockIdx.x + 1) * 3 + k] = b;
   }
+}
+
+// The cell grid of the cloud: cells of half the support radius (plus a
+// twentieth), enlarged when needed so the grid has at most kMaxCells cells,
+// with margins that keep every point's block of cells off the border.
+template<int D>
+__global__ void __launch_bounds__(32)
+    k_na_grid(const double* __restrict__ boxes, double h, double m, double unit_radius,
+              double weight, TankDev* T, uint32_t* id_base) {
+  double lo[3] = {INFINITY, INFINITY, INFINITY};
+  double hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+  for (int b = threadIdx.x; b < kBoxBlocks; b += 32) {
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      lo[k] = fmin(lo[k], boxes[(2 * b) * 3 + k]);
+      hi[k] = fmax(hi[k], boxes[(2 * b + 1) * 3 + k]);
+    }
+  }
+  fold_box<D>(lo, hi);
   if (threadIdx.x != 0) return;
   const double R = unit_radius * h;
-  double cs = R * (1.0 + 1.0 / 65536.0);
+  double cs = 0.5 * R * (1.0 + 1.0 / 20.0);
+  int k_cells = 2;  // cells per radius
   double ext[3];
   for (int k = 0; k < 3; ++k) {
-    ext[k] = k < D ? (s_hi[0][k] - s_lo[0][k]) : 0.0;
+    ext[k] = k < D ? hi[k] - lo[k] : 0.0;
     if (!(ext[k] >= 0.0) || !isfinite(ext[k])) ext[k] = 0.0;
   }
   // Grow the cells (doubling, bounded) until the grid fits; if it never
@@ -122,16 +158,19 @@ __global__ void __launch_bounds__(256)
   for (int it = 0; it < 2100 && !fits && isfinite(cs); ++it) {
     double cells = 1.0;
     for (int k = 0; k < D; ++k) {
-      nc[k] = ceil((ext[k] + 2.0 * (R + cs)) / cs) + 1.0;
+      nc[k] = ceil((ext[k] + 2.0 * (R + 2.0 * cs)) / cs) + 1.0;
       cells *= nc[k];
     }
     fits = cells <= static_cast<double>(kMaxCells);
-    if (!fits) cs *= 2.0;
+    if (!fits) {
+      cs *= 2.0;
+      k_cells = 1;
+    }
   }
   TankDev t{};
   for (int k = 0; k < 3; ++k) {
     const bool use = fits && k < D;
-    t.lo[k] = use ? s_lo[0][k] - (R + cs) : 0.0;
+    t.lo[k] = use ? lo[k] - (R + 2.0 * cs) : 0.0;
     t.nc[k] = use ? static_cast<int32_t>(nc[k]) : 1;
   }
   if (!fits) cs = 1.0;
@@ -146,6 +185,18 @@ __global__ void __launch_bounds__(256)
   t.w = weight * hd;
   t.wg = t.w * t.hinv;
   t.m = m;
+  t.pad = static_cast<uint32_t>(k_cells);
+  // Clipping and culling geometry (tg_particles_upload's formulas); one cell
+  // that holds everything is all border, where neither applies.
+  double extent = 0.0;
+  for (int k = 0; k < D; ++k) extent = fmax(extent, t.nc[k] * cs);
+  const double rc = R * (1.0 + 1.0 / 4096.0);
+  t.cs_f = static_cast<float>(cs);
+  t.inv_cs_f = static_cast<float>(1.0 / cs);
+  t.cull_r2_f = static_cast<float>(rc * rc);
+  t.R_f = static_cast<float>(R);
+  t.list_slack_f = static_cast<float>(extent / 2097152.0 + R / 2048.0);
+  t.band_lo_f = t.R_f;  // positive: the sign marks border cells
   *T = t;
   *id_base = 0;
 }
@@ -165,18 +216,24 @@ __global__ void __launch_bounds__(256)
 
 template<int D>
 __global__ void __launch_bounds__(256)
-    k_na_records(const double* __restrict__ r, const uint32_t* __restrict__ perm,
-                 int64_t n, void* __restrict__ recs, uint32_t* __restrict__ ids) {
+    k_na_records(const double* __restrict__ r, const uint32_t* __restrict__ perm, int64_t n,
+                 const TankDev* __restrict__ T, void* __restrict__ recs,
+                 uint32_t* __restrict__ ids, float* __restrict__ lx, float* __restrict__ ly,
+                 float* __restrict__ lz) {
   const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const uint32_t s = perm[j];
-  if constexpr (D == 2) {
-    static_cast<Pos64_2*>(recs)[j] = Pos64_2{r[int64_t(s) * 2], r[int64_t(s) * 2 + 1]};
-  } else {
-    static_cast<Pos64_3*>(recs)[j] =
-        Pos64_3{r[int64_t(s) * 3], r[int64_t(s) * 3 + 1], r[int64_t(s) * 3 + 2], 0.0};
-  }
+  const double* p = r + static_cast<int64_t>(s) * D;
   ids[j] = s;
+  // lz may be the buffer of perm, whose entry j was read above.
+  lx[j] = __double2float_rn(p[0] - T->lo[0]);
+  ly[j] = __double2float_rn(p[1] - T->lo[1]);
+  if constexpr (D == 2) {
+    static_cast<Pos64_2*>(recs)[j] = Pos64_2{p[0], p[1]};
+  } else {
+    static_cast<Pos64_3*>(recs)[j] = Pos64_3{p[0], p[1], p[2], 0.0};
+    lz[j] = __double2float_rn(p[2] - T->lo[2]);
+  }
 }
 
 template<int D, int K>
@@ -196,7 +253,11 @@ cudaError_t run(unsigned char* base, int64_t n, const double* r, double h,
   const double area = 2.0 * std::sqrt(std::pow(pi, D)) / std::tgamma(D / 2.0);
   const double weight = 1.0 / (kernel_zero_moment(K, D) * area);
   const unsigned g = static_cast<unsigned>((n + 255) / 256);
-  k_na_grid<D><<<1, 256, 0, s>>>(r, n, h, m, kernel_unit_radius(K), weight, T, id_base);
+  // The partial boxes lie where the cell table's bounds come later.
+  static_assert(sizeof(double) * 6 * kBoxBlocks <= kBoundsBytes, "partial boxes");
+  auto* boxes = reinterpret_cast<double*>(base + kOffBounds);
+  k_na_box<D><<<kBoxBlocks, 256, 0, s>>>(r, n, boxes);
+  k_na_grid<D><<<1, 32, 0, s>>>(boxes, h, m, kernel_unit_radius(K), weight, T, id_base);
   k_na_keys<D><<<g, 256, 0, s>>>(r, n, T, keys_a);
   bool in_b = false;
   int64_t launches = 0;
@@ -207,12 +268,18 @@ cudaError_t run(unsigned char* base, int64_t n, const double* r, double h,
   const uint32_t* perm = in_b ? vals_b : vals_a;
   e = build_cell_table(sorted, n, 2 * kMaxCells, cells, base + kOffBounds, s, &launches);
   if (e != cudaSuccess) return e;
-  k_na_records<D><<<g, 256, 0, s>>>(r, perm, n, recs, ids);
+  // The sort's other buffers, and the permutation's own, take the local
+  // coordinates.
+  auto* lx = reinterpret_cast<float*>(in_b ? keys_a : keys_b);
+  auto* ly = reinterpret_cast<float*>(in_b ? vals_a : vals_b);
+  auto* lz = reinterpret_cast<float*>(in_b ? vals_b : vals_a);
+  k_na_records<D><<<g, 256, 0, s>>>(r, perm, n, T, recs, ids, lx, ly, lz);
   // One tank whose first cell (and first id) is 0: id_base doubles as the
   // tank cell-offset table.
-  CloudArgs<D> a{recs, ids, sorted, cells, T, id_base, 1, n, 1, rho, counts, hashes,
-                 id_base};
-  k_sumdens<D, K, false><<<static_cast<unsigned>((n + 127) / 128), 128, 0, s>>>(a);
+  const CloudArgs<D> a{recs, {lx, ly, lz}, nullptr, ids, sorted, cells, T, id_base, 1, n, 0,
+                       rho,  counts,       hashes,  id_base};
+  k_density64<D, K><<<static_cast<unsigned>((32 * n + kDensityBlock - 1) / kDensityBlock),
+                      kDensityBlock, 0, s>>>(a);
   return cudaGetLastError();
 }
 

@@ -585,6 +585,19 @@ __device__ __forceinline__ double rcp_seed(double x) {
   return y;
 }
 
+// 1 / x and sqrt(x), from the hardware seeds by one third-order iteration.
+__device__ __forceinline__ double rcp_f64(double x) {
+  const double y = rcp_seed(x);
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double sqrt_f64(double x) {
+  const double y = rsqrt_seed(x);
+  const double r = x * y;
+  const double e = fma(-r, y, 1.0);
+  return __double2hiint(x) == 0 ? 0.0 : fma(r, e * fma(e, 0.375, 0.5), r);
+}
+
 __device__ __forceinline__ Dat32 load_dat_wide(const Dat32* p, uint32_t j) {
   Dat32 r;
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"

@@ -79,19 +79,6 @@ __device__ __forceinline__ void list_entries(const ListArgs<D, F>& A, int64_t i,
   }
 }
 
-// 1 / x and sqrt(x), from the hardware seeds by one third-order iteration.
-__device__ __forceinline__ double rcp_f64(double x) {
-  const double y = rcp_seed(x);
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-__device__ __forceinline__ double sqrt_f64(double x) {
-  const double y = rsqrt_seed(x);
-  const double r = x * y;
-  const double e = fma(-r, y, 1.0);
-  return __double2hiint(x) == 0 ? 0.0 : fma(r, e * fma(e, 0.375, 0.5), r);
-}
-
 template<int Team>
 __device__ __forceinline__ double team_sum(double v) {
 #pragma unroll
