@@ -48,9 +48,9 @@ def _jittered(scn, amount=0.1, seed=3):
 
 
 # 16, 4 and 1 lanes per particle: fluid counts on both sides of the limits
-# (a quarter of 512 particles per multiprocessor, and 512).
-@pytest.mark.parametrize("dim,nx", ((2, 11), (2, 98), (2, 101), (2, 196), (2, 199), (3, 9),
-                                    (3, 23), (3, 36)))
+# (32 and 128 particles per multiprocessor; 152 of them).
+@pytest.mark.parametrize("dim,nx", ((2, 11), (2, 49), (2, 50), (2, 98), (2, 99), (2, 199), (3, 9),
+                                    (3, 15), (3, 23)))
 def test_list_widths(gpu_lib, dim, nx):
     scn = (scenarios.dam_break_2d(nx_per_H=nx) if dim == 2
            else scenarios.dam_break_3d(nx_per_H=nx, column=(1.7, 1.0, 1.0)))

@@ -541,13 +541,18 @@ class Engine final : public EngineBase {
   }
 
   // Lanes per target of the list passes: one where the particles alone give
-  // every multiprocessor 16 warps, more for smaller runs (4 entries of the
-  // list per lane and turn, so 16 lanes take a 2D list at once).  A launch
-  // shape that asks for several lanes gets at least 4.
+  // every multiprocessor four warps, 4 and 16 for smaller runs, whose passes
+  // are chains of latencies (a lane takes 4 entries of the list per turn, so
+  // 16 lanes take a 2D list at once).  More lanes repeat the update's FP64
+  // operations for fewer particles per warp.  Measured in us per pass, 16 / 4
+  // / 1 lanes: 800 fluid particles FP64 with shifting, 1 step 292 / 397 / 722;
+  // 12,800 FP64, 10 steps 4426 / 3965 / 4489; 62,000 compensated with
+  // shifting, 4 steps - / 3311 / 3200.  A launch shape that asks for several
+  // lanes gets at least 4.
   static int list_team(const Context& C) {
-    const int64_t full = 512 * static_cast<int64_t>(C.sm_count > 0 ? C.sm_count : 152);
-    if (4 * C.n_fluid < full) return 16;
-    return C.n_fluid < full || C.force_team > 1 ? 4 : 1;
+    const int64_t warps = 4 * static_cast<int64_t>(C.sm_count > 0 ? C.sm_count : 152);
+    if (C.n_fluid < 8 * warps) return 16;
+    return C.n_fluid < 32 * warps || C.force_team > 1 ? 4 : 1;
   }
   template<int Team>
   void launch_build(Context& C, const ListArgs<D, F>& A) {

@@ -113,17 +113,20 @@ __device__ __forceinline__ void get_coords(const Dat32& r, int* q) {
 
 // Records: tank constants of a fluid particle (common to the gather and the
 // stages), and their stores.
+// The plain form's pad word holds the potential H(rho) of a tank with walls,
+// once per particle instead of once per wall and neighbour.
 template<int D>
 __device__ __forceinline__ Dat64 fluid_record(const PhysDev& P, const TankDev& T, const double* v,
-                                              double rho) {
+                                              double rho, bool walls) {
   double pr, c;
   tait_f64(P, T, rho, pr, c);
   const double inv = 1.0 / rho;
-  return Dat64{v[0], v[1], D == 3 ? v[2] : 0.0, rho, pr * inv * inv, c, inv, 0.0};
+  return Dat64{v[0], v[1], D == 3 ? v[2] : 0.0, rho, pr * inv * inv, c, inv,
+               walls ? potential_f64(P, T, rho) : 0.0};
 }
 template<int D>
 __device__ __forceinline__ Dat32 fluid_record(const PhysDev& P, const TankDev& T, const float* v,
-                                              float rho) {
+                                              float rho, bool) {
   float pr, c;
   tait_f32(P, T, rho, pr, c);
   const float inv = __frcp_rn(T.rho0_f + rho);
@@ -194,7 +197,7 @@ __global__ void __launch_bounds__(256) k_list_gather(ListArgs<D, F> A) {
       }
       const R rho = S.X.rho[src];
       S.Udst.rho[j] = rho;
-      rec = fluid_record<D>(S.phys, T, v, rho);
+      rec = fluid_record<D>(S.phys, T, v, rho, A.n_walls > 0);
       R a2 = R(0), v2 = R(0);
 #pragma unroll
       for (int k = 0; k < D; ++k) {
@@ -292,7 +295,7 @@ __global__ void __launch_bounds__(256) k_list_select(ListArgs<D, F> A) {
 
 struct ListRows {
   int y0, y1, z0, z1, x0, x1;  // the block of cells
-  int yb, zb, span;            // its unclipped corner and width
+  int x, yb, zb, span;         // its centre, unclipped corner and width
   float RL, RL2;
   bool border;
 };
@@ -308,6 +311,7 @@ __device__ __forceinline__ ListRows list_rows(const TankDev& T, const int* c, co
   W.border = c[0] - kk <= 0 || c[0] + kk >= T.nc[0] - 1 || c[1] - kk <= 0 ||
              c[1] + kk >= T.nc[1] - 1;
   if constexpr (D == 3) W.border = W.border || c[2] - kk <= 0 || c[2] + kk >= T.nc[2] - 1;
+  W.x = c[0];
   W.yb = c[1] - kk;
   W.zb = D == 3 ? c[2] - kk : 0;
   W.span = 2 * kk + 1;
@@ -406,8 +410,7 @@ struct ListWriter {
   }
 };
 
-// The list of slot i, by Team lanes (lane tl of the team; the lanes split
-// the rows).  Wall targets list fluid entries only.  A warp with a border target
+// The list of slot i, by Team lanes (lane tl of the team).  Wall targets list fluid entries only.  A warp with a border target
 // takes the FP64 test for all its targets: kept apart, so that the common
 // loop holds no FP64 instruction (selected per candidate, they issued for
 // every candidate and the build of 2M particles took 9.2 ms).
@@ -463,24 +466,24 @@ __device__ __forceinline__ void build_list(const ListArgs<D, F>& A, const TankDe
     w.finish();
     cnt = w.cnt;
   } else {
-    const int ny = W.y1 - W.y0 + 1;
-    const int rows = ny > 0 ? ny * (W.z1 - W.z0 + 1) : 0;
-    int t = tl;
-    uint32_t j = 0, e = 0;
-    const unsigned below = tmask & ((1u << (threadIdx.x & 31u)) - 1u);
-    for (;;) {
-      while (j >= e && t < rows) {
-        list_row<D>(T, W, xl, S.cell_start, W.y0 + t % ny, W.z0 + t / ny, j, e);
-        t += Team;
-      }
-      const bool have = j < e;
-      if (__ballot_sync(0xffffffffu, have) == 0u) break;
-      const bool acc = have && accept(A.lrec[have ? j : 0u], j);
-      const unsigned hit = __ballot_sync(0xffffffffu, acc);
-      const uint32_t p = cnt + __popc(hit & below);
-      if (acc && p < cap) A.list[list_at(i, p, A.cap)] = j;
-      cnt += __popc(hit & tmask);
-      if (have) ++j;
+    // The team's lanes share every row; lanes without a target sit out.
+    if (target) {
+      const int c[3] = {W.x, W.yb + (W.span >> 1), D == 3 ? W.zb + (W.span >> 1) : 0};
+      const float o[3] = {xl[0] - static_cast<float>(c[0]) * T.cs_f,
+                          xl[1] - static_cast<float>(c[1]) * T.cs_f,
+                          D == 3 ? xl[2] - static_cast<float>(c[2]) * T.cs_f : 0.f};
+      const unsigned below = tmask & ((1u << (threadIdx.x & 31u)) - 1u);
+      for_shared_rows<D, Team>(T, c, W.span >> 1, S.cell_start, tl, tmask, Border ? nullptr : o,
+                               W.RL2, [&](uint32_t s, uint32_t e) {
+        for (uint32_t j0 = s; j0 < e; j0 += Team) {
+          const uint32_t j = j0 + tl;
+          const bool acc = j < e && accept(A.lrec[j < e ? j : s], j);
+          const unsigned hit = __ballot_sync(tmask, acc) & tmask;
+          const uint32_t p = cnt + __popc(hit & below);
+          if (acc && p < cap) A.list[list_at(i, p, A.cap)] = j;
+          cnt += __popc(hit);
+        }
+      });
     }
   }
   if (target && tl == 0) {
@@ -495,7 +498,7 @@ __device__ __forceinline__ void build_lists(const ListArgs<D, F>& A, int64_t i, 
                                             int tl, unsigned tmask) {
   const StageArgs<D, F>& S = A.S;
   const TankDev* T = S.tanks;
-  ListRows W{0, -1, 0, -1, 0, 0, 0, 0, 0, 0.f, 0.f, false};
+  ListRows W{0, -1, 0, -1, 0, 0, 0, 0, 0, 0, 0.f, 0.f, false};
   float xl[3] = {0.f, 0.f, 0.f};
   if (target) {
     const uint32_t key = S.skey[i];
@@ -820,6 +823,21 @@ struct ListPairF64 {
 };
 
 // ---------------------------------------------------------------------------
+// rho(H) of the Tait law with xi = 7, rho0 u^(1/6) with u = 1 + 6 H / cs0^2:
+// the FP32 power y0 (relative error below 2^-19) times the binomial series
+// of (u / y0^6)^(1/6) to second order (truncation below 2^-57), 14 FP64
+// operations in a chain instead of pow's.
+__device__ __forceinline__ double wall_density_f64(const PhysDev& P, const TankDev& T, double H) {
+  if (!P.xi_is_7 || P.eos != TG_EOS_TAIT) return density_from_potential_f64(P, T, H);
+  const double u = 1.0 + 6.0 * H / (T.cs0 * T.cs0);
+  // FP32's range with room for its powers (false for a NaN as well).
+  if (!(u > 1e-30 && u < 1e30)) return density_from_potential_f64(P, T, H);
+  const double y0 = static_cast<double>(powf(static_cast<float>(u), 1.f / 6.f));
+  const double y2 = y0 * y0, y6 = y2 * y2 * y2;
+  const double e = (u - y6) * rcp_f64(y6);
+  return T.rho0 * fma(y0, e * fma(e, -5.0 / 72.0, 1.0 / 6.0), y0);
+}
+
 // Wall extrapolation (k_walls) over the walls' lists: teams of 8 lanes take
 // the listed walls in turn, the lanes the list's groups of four entries.
 constexpr int kListWallTeam = 8;
@@ -856,12 +874,11 @@ __global__ void __launch_bounds__(128) k_list_walls(ListArgs<D, F> A) {
           const double s2 = dist2_exact<D>(pb, pe, d);
           if (s2 > T.radius2) continue;
           const Dat64 b = load_dat(A.dat_in, js[q]);
-          const double W = T.w * KernelPoly<K>::value(sqrt(s2) * T.hinv);
-          double Hb = potential_f64(S.phys, T, b.rho);
+          const double VW = b.invrho * KernelPoly<K>::value(sqrt_f64(s2) * T.hinv);
+          double Hb = b.pad;
           if (S.fc.on) Hb += S.phys.g * dot_d<D>(d, ne) * ne[1];
-          const double VW = T.m * b.invrho * W;
           Ss += VW;
-          H += VW * Hb;
+          H = fma(VW, Hb, H);
         }
       }
 #pragma unroll
@@ -870,8 +887,8 @@ __global__ void __launch_bounds__(128) k_list_walls(ListArgs<D, F> A) {
         H += __shfl_xor_sync(tmask, H, o, kListWallTeam);
       }
       if (tl == 0) {
-        const double Hs = fabs(Ss) <= 6.0554544523933395e-06 ? 0.0 : H / Ss;
-        A.dat_in[ew] = wall_record<D>(S.phys, T, density_from_potential_f64(S.phys, T, Hs), true);
+        const double Hs = fabs(Ss * (T.m * T.w)) <= 6.0554544523933395e-06 ? 0.0 : H / Ss;
+        A.dat_in[ew] = wall_record<D>(S.phys, T, wall_density_f64(S.phys, T, Hs), true);
       }
     } else {
       const float hq = T.list_hq_f;
@@ -1031,7 +1048,7 @@ __device__ __forceinline__ void list_epilogue(const ListArgs<D, F>& A, int64_t i
       cell_of<D>(T, pn, cn, outside);
       A.curkey[i] = key_of(flat_cell<D>(T, cn), false);
     }
-    store_list_record<D>(A.pos_out, A.dat_out, i, T, pn, fluid_record<D>(S.phys, T, vn, rn));
+    store_list_record<D>(A.pos_out, A.dat_out, i, T, pn, fluid_record<D>(S.phys, T, vn, rn, A.n_walls > 0));
     return;
   }
   int c[3] = {0, 0, 0};
