@@ -102,3 +102,21 @@ def test_particles_outside_the_grid(gpu_lib, dim):
         r[n // 8: n // 4, 1] += 1.3 * (hi - lo)
 
     _check(scn, physics.baseline_params(dim), 2, move)
+
+
+@pytest.mark.parametrize("dim", (2, 3))
+@pytest.mark.parametrize("steps", (1, 2, 3, 5))
+def test_chained_steps(gpu_lib, dim, steps):
+    # The compensated form's steps share their lists in pairs; tanks of
+    # different time steps, odd counts, and the time of every tank.
+    scn = (scenarios.batched_tanks(n_tanks=4, n_range=(8, 21), seed=7) if dim == 2
+           else scenarios.batched_tanks_3d(n_tanks=3, n_range=(5, 9), seed=7))
+    scn = _jittered(scn)
+    P = physics.baseline_params(dim)
+    _check(scn, P, steps)
+    o = oracle_run(scn, P, steps)
+    P.precision = _abi.TG_FP32C
+    with gpu_context(scn, P) as ctx:
+        dt = ctx.step(steps)
+        np.testing.assert_allclose(ctx.time(), o.time, rtol=2e-6)
+        np.testing.assert_allclose(dt, o.dt, rtol=2e-6)

@@ -80,9 +80,11 @@ void Context::release_all() {
 }
 
 void Context::invalidate_graph() {
-  for (cudaGraphExec_t& g : graph_exec) {
-    if (g != nullptr) cudaGraphExecDestroy(g);
-    g = nullptr;
+  for (auto& per_length : graph_exec) {
+    for (cudaGraphExec_t& g : per_length) {
+      if (g != nullptr) cudaGraphExecDestroy(g);
+      g = nullptr;
+    }
   }
 }
 
@@ -600,7 +602,7 @@ int upload_particles(tg_context* ctx, int32_t n_tanks, const tg_tank* tanks,
   TG_CUDA(&C, A(C.d_id_base, sizeof(uint32_t) * n_tanks));
   TG_CUDA(&C, A(C.d_wall_from, sizeof(uint32_t) * n_tanks));
   TG_CUDA(&C, A(C.d_tank_of, sizeof(uint32_t) * nn));
-  TG_CUDA(&C, A(C.d_dt, sizeof(double) * n_tanks));
+  TG_CUDA(&C, A(C.d_dt, sizeof(double) * n_tanks * tg::kListChain));
   TG_CUDA(&C, A(C.d_dt_last, sizeof(double) * n_tanks));
   TG_CUDA(&C, A(C.d_time, sizeof(double) * n_tanks));
   TG_CUDA(&C, A(C.d_err, 4 * sizeof(uint32_t)));
@@ -636,7 +638,7 @@ int upload_particles(tg_context* ctx, int32_t n_tanks, const tg_tank* tanks,
     for (int64_t i = 0; i < nt; ++i) tank_of[base + i] = static_cast<uint32_t>(t);
     base += nt;
   }
-  std::vector<double> inf(static_cast<size_t>(n_tanks),
+  std::vector<double> inf(static_cast<size_t>(n_tanks) * tg::kListChain,
                           std::numeric_limits<double>::infinity());
   std::vector<double> zeros(static_cast<size_t>(n_tanks), 0.0);
   cudaStream_t s = C.stream;
@@ -653,7 +655,7 @@ int upload_particles(tg_context* ctx, int32_t n_tanks, const tg_tank* tanks,
                               sizeof(uint32_t) * n_tanks, cudaMemcpyHostToDevice, s));
   TG_CUDA(&C, cudaMemcpyAsync(C.d_tank_of, tank_of.data(), sizeof(uint32_t) * nn,
                               cudaMemcpyHostToDevice, s));
-  TG_CUDA(&C, cudaMemcpyAsync(C.d_dt, inf.data(), sizeof(double) * n_tanks,
+  TG_CUDA(&C, cudaMemcpyAsync(C.d_dt, inf.data(), sizeof(double) * inf.size(),
                               cudaMemcpyHostToDevice, s));
   TG_CUDA(&C, cudaMemcpyAsync(C.d_dt_last, zeros.data(), sizeof(double) * n_tanks,
                               cudaMemcpyHostToDevice, s));
@@ -738,37 +740,39 @@ namespace {
 // while profiling, without graphs, or where a stopped step is repeated.
 int enqueue_steps(Context& C, int32_t n, bool direct) {
   TG_CUDA(&C, C.engine->ensure_keys(C));
-  if (direct) {
-    for (int32_t i = 0; i < n; ++i) {
-      TG_CUDA(&C, C.engine->enqueue_step(C));
-      C.prof.stages += tg::force_passes(C.P.integrator);
-      C.prof.forces_launches += tg::force_passes(C.P.integrator);
+  const int chain = C.engine->chain(C);
+  for (int32_t i = 0; i < n;) {
+    const int steps = chain > 1 && n - i >= chain ? chain : 1;
+    i += steps;
+    if (direct) {
+      TG_CUDA(&C, C.engine->enqueue_step(C, steps));
+      C.prof.stages += steps * tg::force_passes(C.P.integrator);
+      C.prof.forces_launches += steps * tg::force_passes(C.P.integrator);
+      continue;
     }
-    return TG_OK;
-  }
-  for (int32_t i = 0; i < n; ++i) {
     // The re-sort is taken only in the home order of an earlier sort, a
     // host-side choice baked into the graph: one graph for each.
-    const int g = C.order_valid ? 1 : 0;
-    if (C.graph_exec[g] == nullptr) {
+    const int l = steps > 1 ? 1 : 0, o = C.order_valid ? 1 : 0;
+    cudaGraphExec_t& exec = C.graph_exec[l][o];
+    if (exec == nullptr) {
       cudaGraph_t graph = nullptr;
       const int64_t before = C.launches;
       TG_CUDA(&C, cudaStreamBeginCapture(C.stream, cudaStreamCaptureModeThreadLocal));
-      const cudaError_t e = C.engine->enqueue_step(C);
+      const cudaError_t e = C.engine->enqueue_step(C, steps);
       const cudaError_t e2 = cudaStreamEndCapture(C.stream, &graph);
       if (e != cudaSuccess) return cuda_fail(&C, e, "enqueue_step");
       if (e2 != cudaSuccess) return cuda_fail(&C, e2, "cudaStreamEndCapture");
-      C.graph_kernels[g] = C.launches - before;
+      C.graph_kernels[l][o] = C.launches - before;
       C.launches = before;
-      const cudaError_t e3 = cudaGraphInstantiate(&C.graph_exec[g], graph, 0);
+      const cudaError_t e3 = cudaGraphInstantiate(&exec, graph, 0);
       cudaGraphDestroy(graph);
       if (e3 != cudaSuccess) {
-        C.graph_exec[g] = nullptr;
+        exec = nullptr;
         return cuda_fail(&C, e3, "cudaGraphInstantiate");
       }
     }
-    TG_CUDA(&C, cudaGraphLaunch(C.graph_exec[g], C.stream));
-    C.launches += C.graph_kernels[g];
+    TG_CUDA(&C, cudaGraphLaunch(exec, C.stream));
+    C.launches += C.graph_kernels[l][o];
     C.keys_valid = true;
     C.order_valid = true;
   }

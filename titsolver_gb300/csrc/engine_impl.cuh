@@ -86,6 +86,7 @@ class Engine final : public EngineBase {
     }
     posrec_b_ = nullptr;
     datrec_b_ = nullptr;
+    travel_ = nullptr;
     // Two spare records: the staged force pass copies row segments rounded
     // out to 16-byte boundaries, which may reach one record past the end.
     A(posrec_, n + 2);
@@ -135,7 +136,7 @@ class Engine final : public EngineBase {
       double most = 0.0;
       for (size_t t = 0; t < C.tanks.size(); ++t) {
         const TankDev& T = C.tankdev[t];
-        const double R = 1.06 * T.R_f;
+        const double R = (F == TG_FP32C ? 1.1 : 1.06) * T.R_f;
         const double ball = D == 2 ? 3.14159265358979 * R * R : 4.18879020478639 * R * R * R;
         most = std::max(most, ball * T.rho0 / T.m);
         // Tank-local FP32 coordinates must resolve the radius.
@@ -163,6 +164,8 @@ class Engine final : public EngineBase {
         e = C.alloc(reinterpret_cast<void**>(&datrec_b_), sizeof(DatRec) * (C.n + kListScan));
         if (e == cudaSuccess && F == TG_FP64) {
           e = C.alloc(reinterpret_cast<void**>(&posrec_b_), sizeof(PosRec) * C.n);
+        } else if (e == cudaSuccess) {
+          e = C.alloc(reinterpret_cast<void**>(&travel_), sizeof(float) * C.n);
         }
       }
       if (e != cudaSuccess) {
@@ -175,9 +178,18 @@ class Engine final : public EngineBase {
     return cudaSuccess;
   }
 
-  cudaError_t enqueue_step(Context& C) override {
+  int chain(const Context& C) const override {
+    // Not where the lists would serve the FP64 pipe, which pays for every
+    // entry, nor after a step of this context had to be repeated.
+    return F == TG_FP32C && C.lists && C.list_redos == 0 &&
+                   C.P.post_integrate != TG_POST_SHIFTING && !C.faces.on
+               ? kListChain
+               : 1;
+  }
+
+  cudaError_t enqueue_step(Context& C, int steps) override {
     if (C.n == 0) return cudaSuccess;
-    if (C.lists) return enqueue_list_step(C);
+    if (C.lists) return enqueue_list_step(C, steps);
     static const double w3[3] = {1.0, 1.0 / 4.0, 2.0 / 3.0};
     static const double w2[2] = {1.0, 1.0 / 2.0};
     const int integ = C.P.integrator;
@@ -231,7 +243,7 @@ class Engine final : public EngineBase {
       cudaError_t e = enqueue_post(C);
       if (e != cudaSuccess) return e;
     }
-    return step_end(C);
+    return step_end(C, 1);
   }
 
   cudaError_t enqueue_prepare(Context& C) override {
@@ -373,10 +385,10 @@ class Engine final : public EngineBase {
     return a;
   }
 
-  cudaError_t step_end(Context& C) {
+  cudaError_t step_end(Context& C, int steps) {
     const int tok = C.group_begin(kGroupForces);
     k_step_end<<<grid_for(C.ntanks, 128), 128, 0, C.stream>>>(
-        C.d_dt, C.d_dt_last, C.d_time, C.d_vmax, C.d_err, C.ntanks);
+        C.d_dt, C.d_dt_last, C.d_time, C.d_vmax, C.d_err, C.ntanks, steps);
     C.launches += 1;
     C.group_end(tok);
     return cudaGetLastError();
@@ -389,9 +401,9 @@ class Engine final : public EngineBase {
     C.d_list_cnt = nullptr;
   }
 
-  // One step on neighbour lists (pairlist.cuh): one sort, lists for its
+  // Steps on neighbour lists (pairlist.cuh): one sort, lists for all their
   // stages, and per stage the wall pass and the pair sums.
-  cudaError_t enqueue_list_step(Context& C) {
+  cudaError_t enqueue_list_step(Context& C, int steps) {
     cudaError_t e = enqueue_sort(C);
     if (e != cudaSuccess) return e;
     ListArgs<D, F> A{};
@@ -413,6 +425,8 @@ class Engine final : public EngineBase {
     A.n_walls = C.n_wall;
     A.cap = C.list_cap;
     A.margin = C.list_margin;
+    A.chain = steps;
+    A.dt_build = C.d_dt;
     int tok = C.group_begin(kGroupReorder);
     e = clear_wall_counts(C, S);
     if (e != cudaSuccess) return e;
@@ -437,18 +451,40 @@ class Engine final : public EngineBase {
     static const double w2[2] = {1.0, 1.0 / 2.0};
     const int stages = C.P.integrator == TG_SSPRK2 ? 2 : 3;
     const bool shifting = C.P.post_integrate == TG_POST_SHIFTING;
-    for (int s = 0; s < stages; ++s) {
-      A.first = s == 0;
-      A.last = s == stages - 1 && !shifting;
-      A.post = s == stages - 1 && shifting;
+    // Three position buffers take turns: the step's start, and two for its
+    // stages, of which the last one written is the next step's start.
+    double* const* pos[3] = {Y_.pos, U_[0].pos, U_[1].pos};
+    int start = 0;
+    bool in_b = false;  // which records the stage reads
+    for (int q = 0; q < steps * stages; ++q) {
+      const int step = q / stages, s = q % stages;
+      const bool end = s == stages - 1;  // of its step
+      if (s == 0) {
+        for (int k = 0; k < D; ++k) A.S.Y.pos[k] = pos[start][k];
+        A.S.Udst = U_[step & 1];
+        A.S.dt = C.d_dt + static_cast<size_t>(step) * C.ntanks;
+        A.travel = step > 0 ? travel_ : nullptr;
+      }
+      A.first = q == 0;
+      A.carry = end && step + 1 < steps;
+      A.last = end && !A.carry && !shifting;
+      A.post = end && shifting;
+      if (A.carry) {
+        A.next = U_[(step + 1) & 1];
+        A.dt_next = A.S.dt + C.ntanks;
+        A.travel_out = travel_;
+      }
       A.S.lincomb = s > 0;
       A.S.w_new = (stages == 2 ? w2 : w3)[s];
       A.w0 = 1.0 - A.S.w_new;
       A.wr = static_cast<R>(A.S.w_new);
       A.w0r = static_cast<R>(A.w0);
-      A.pos_out = reinterpret_cast<typename ListArgs<D, F>::PosRec*>(s == 1 ? posrec_ : posrec_b_);
-      A.dat_out = s == 1 ? datrec_ : datrec_b_;
-      for (int k = 0; k < D; ++k) A.pout[k] = U_[s & 1].pos[k];
+      A.pos_out = reinterpret_cast<typename ListArgs<D, F>::PosRec*>(in_b ? posrec_ : posrec_b_);
+      A.dat_out = in_b ? datrec_ : datrec_b_;
+      in_b = !in_b;
+      const int out = (start + 1 + (s & 1)) % 3;
+      for (int k = 0; k < D; ++k) A.pout[k] = pos[out][k];
+      if (end) start = out;
       if (C.n_wall > 0) {
         tok = C.group_begin(kGroupWalls);
         const StageArgs<D, F> a = list_stage_view(A);
@@ -510,7 +546,7 @@ class Engine final : public EngineBase {
     }
     C.keys_valid = true;
     C.order_valid = true;
-    return step_end(C);
+    return step_end(C, steps);
   }
 
   // The face passes' view of a stage: its positions and records, and (past
@@ -825,6 +861,7 @@ class Engine final : public EngineBase {
   DatRec* datrec_ = nullptr;
   PosRec* posrec_b_ = nullptr;  // the list step's second records
   DatRec* datrec_b_ = nullptr;
+  float* travel_ = nullptr;     // paths within a chain of steps
 };
 
 template <int D, int F, int K>

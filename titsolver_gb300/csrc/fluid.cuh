@@ -2332,24 +2332,27 @@ __global__ void __launch_bounds__(256)
   if (drho != nullptr) drho[id] = X.drho[i];
 }
 
-// End of step: advance per-tank time, keep dt, reset the reductions, count
-// the step.  status: the error word, the stop word, the steps finished; a
-// stopped step advances nothing.
-static __global__ void k_step_end(double* dt, double* dt_last, double* time, unsigned* vmax,
-                                  uint32_t* status, int ntanks) {
+// End of a step, or of a chain of steps (dt: ntanks per step): advance
+// per-tank time, keep dt, reset the reductions, count the steps.  status: the
+// error word, the stop word, the steps finished; a stop advances nothing.
+static __global__ void k_step_end(double* dts, double* dt_last, double* time, unsigned* vmax,
+                                  uint32_t* status, int ntanks, int steps) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const bool done = status[1] == 0u;
-  if (t == 0 && done) status[2] += 1u;
+  if (t == 0 && done) status[2] += static_cast<uint32_t>(steps);
   if (t >= ntanks) return;
   uint32_t* err = status;
   vmax[t] = 0u;
-  const double d = dt[t];
-  if (done && isfinite(d)) {
-    if (!(d > 0.0)) atomicOr(err, static_cast<uint32_t>(TG_DEV_BAD_DT));
-    time[t] += d;
-    dt_last[t] = d;
+  for (int q = 0; q < steps; ++q) {
+    double* dt = dts + static_cast<size_t>(q) * ntanks;
+    const double d = dt[t];
+    if (done && isfinite(d)) {
+      if (!(d > 0.0)) atomicOr(err, static_cast<uint32_t>(TG_DEV_BAD_DT));
+      time[t] += d;
+      dt_last[t] = d;
+    }
+    dt[t] = __longlong_as_double(0x7ff0000000000000ll);
   }
-  dt[t] = __longlong_as_double(0x7ff0000000000000ll);
 }
 
 }  // namespace tg

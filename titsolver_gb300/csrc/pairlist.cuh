@@ -20,6 +20,11 @@
 // repeats the step with a sort per stage (tg_step).  Nothing is approximated:
 // the predicate |r_ab| <= R is applied to every entry in every stage.
 //
+// Chains.  The compensated form's steps within one tg_step call share the
+// lists (kListChain at a time): the lists are as much wider, and the first
+// step's last stage hands its state on in the records.  The home state
+// is written by the chain's last step, so a stop repeats the whole chain.
+//
 // Positions of the compensated form are 32-bit fixed point, in units of
 // 2^-28 cells modulo 2^32: a difference is exact while it is below 8 cells
 // (listed pairs are within R + 2 delta <= 1.5 R <= 4.5 cells), whatever the
@@ -63,6 +68,17 @@ struct ListArgs {
   int cap;                // entries per slot, a multiple of 4
   float margin;           // acceleration share of delta, in R
   int first, last;
+  // Chains: steps that share the lists.  dt_build: the first step's dt (S.dt:
+  // the present step's).  carry: the last stage of a step that another one
+  // follows, which leaves its state as that step's start (positions in pout,
+  // velocity and density in next) and folds its time step into dt_next.
+  int chain, carry;
+  const double* dt_build;
+  double* dt_next;
+  StartBuf<R> next;
+  float* travel;          // path since the build up to the present step's
+                          // start, or null in the first step
+  float* travel_out;
   int post;               // the last stage of a step with post-integration:
                           // keeps the rates in Y and leaves X to that
   double w0;              // 1 - S.w_new, and both in the form's type
@@ -78,8 +94,10 @@ __device__ __forceinline__ size_t list_at(int64_t s, uint32_t p, int cap) {
 // The displacement bound of a tank's particles in this step.
 template<int D, int F>
 __device__ __forceinline__ float list_delta(const ListArgs<D, F>& A, const TankDev& T,
-                                            uint32_t tk, float dt) {
-  const float d = dt * __uint_as_float(A.vmax[tk]) * 1.0001f + A.margin * T.R_f;
+                                            uint32_t tk) {
+  const float d = static_cast<float>(A.chain) *
+                  (static_cast<float>(A.dt_build[tk]) * __uint_as_float(A.vmax[tk]) * 1.0001f +
+                   A.margin * T.R_f);
   return fminf(d, 0.25f * T.R_f);  // also for a tank without fluid (dt = inf)
 }
 
@@ -154,6 +172,30 @@ __device__ __forceinline__ void store_list_record(const int4*, Dat32* dat, int64
   dat[j] = rec;
 }
 
+// FluidEquations::compute_time_step (fluid_equations.hpp:205-230) of one
+// particle, compensated form.
+__device__ __forceinline__ float time_step(const PhysDev& P, const TankDev& T, float speed,
+                                           float accel, float drho, float c) {
+  const float h = T.h_f;
+  const float dt_ac = P.cfl_f * h / (c + speed);
+  const float dt_vi = P.c_visc_f * h * h * (T.rho0_f + drho) / P.mu_f;
+  const float dt_fo = P.c_force_f * sqrtf(h / fmaxf(accel, P.g_f));
+  return fminf(dt_ac, fminf(dt_vi, dt_fo));
+}
+
+// Minimum over a tank, from the lanes that are here: one atomic for those of
+// one tank, and only where it would lower the result.
+__device__ __forceinline__ void fold_time_step(double* dt, uint32_t tk, float mine) {
+  const unsigned here = __activemask();
+  int same = 0;
+  __match_all_sync(here, tk, &same);
+  unsigned bits = __float_as_uint(mine);  // positive floats order like their bits
+  if (same) bits = __reduce_min_sync(here, bits);
+  if (same && static_cast<int>(threadIdx.x & 31u) != __ffs(here) - 1) return;
+  const double d = static_cast<double>(__uint_as_float(bits));
+  if (d < *static_cast<volatile double*>(dt + tk)) atomic_min_pos(dt + tk, d);
+}
+
 // ---------------------------------------------------------------------------
 // Gather into cell order.
 template<int D, int F>
@@ -214,12 +256,8 @@ __global__ void __launch_bounds__(256) k_list_gather(ListArgs<D, F> A) {
         dt_a = fmin(dt_ac, fmin(dt_vi, dt_fo));
         v_a = __double2float_ru(speed);
       } else {
-        const float h = T.h_f, speed = sqrtf(v2);
-        const float rhof = T.rho0_f + rho;
-        const float dt_ac = S.phys.cfl_f * h / (rec.c + speed);
-        const float dt_vi = S.phys.c_visc_f * h * h * rhof / S.phys.mu_f;
-        const float dt_fo = S.phys.c_force_f * sqrtf(h / fmaxf(sqrtf(a2), S.phys.g_f));
-        dt_a = static_cast<double>(fminf(dt_ac, fminf(dt_vi, dt_fo)));
+        const float speed = sqrtf(v2);
+        dt_a = static_cast<double>(time_step(S.phys, T, speed, sqrtf(a2), rho, rec.c));
         v_a = speed;
       }
     }
@@ -272,7 +310,7 @@ __global__ void __launch_bounds__(256) k_list_select(ListArgs<D, F> A) {
     const float4 x = A.lrec[e];
     const float xl[3] = {x.x, x.y, x.z};
     const float reach = sqrtf(T.wall_skip_r2_f) +
-                        2.f * list_delta(A, T, tk, static_cast<float>(S.dt[tk]));
+                        2.f * list_delta(A, T, tk);
     act = !beyond_fluid<D>(S.fbox, S.ntanks, tk, reach * reach, xl);
   }
   const unsigned mask = __ballot_sync(0xffffffffu, act);
@@ -510,8 +548,7 @@ __device__ __forceinline__ void build_lists(const ListArgs<D, F>& A, int64_t i, 
     xl[0] = x.x;
     xl[1] = x.y;
     xl[2] = x.z;
-    W = list_rows<D>(*T, c, xl, T->R_f + T->list_slack_f +
-                          2.f * list_delta(A, *T, tk, static_cast<float>(S.dt[tk])));
+    W = list_rows<D>(*T, c, xl, T->R_f + T->list_slack_f + 2.f * list_delta(A, *T, tk));
   }
   if (__any_sync(0xffffffffu, W.border)) {
     build_list<D, F, Team, Wall, true>(A, *T, W, xl, i, target, tl, tmask);
@@ -1027,12 +1064,13 @@ __device__ __forceinline__ void list_epilogue(const ListArgs<D, F>& A, int64_t i
   }
   if (!A.last) {
     float d2 = 0.f;
+    if (A.post || A.carry) {
+#pragma unroll
+      for (int k = 0; k < D; ++k) dis[k] = __double2float_rn(pn[k] - S.Y.pos[k][i]);
+    }
     if (A.post) {
 #pragma unroll
-      for (int k = 0; k < D; ++k) {
-        dis[k] = __double2float_rn(pn[k] - S.Y.pos[k][i]);
-        S.Y.dv[k][i] = dv[k];
-      }
+      for (int k = 0; k < D; ++k) S.Y.dv[k][i] = dv[k];
       S.Y.drho[i] = drho;
     }
 #pragma unroll
@@ -1040,15 +1078,31 @@ __device__ __forceinline__ void list_epilogue(const ListArgs<D, F>& A, int64_t i
       d2 = fmaf(dis[k], dis[k], d2);
       A.pout[k][i] = pn[k];
     }
-    const float delta = list_delta(A, T, tk, dtf);
-    if (!(d2 <= delta * delta)) atomicOr(A.stop, kStopMoved);
+    float far = sqrtf(d2);
+    if (A.travel != nullptr) far += A.travel[i];
+    if (!(far <= list_delta(A, T, tk))) atomicOr(A.stop, kStopMoved);
     if (A.curkey != nullptr) {
       int cn[3] = {0, 0, 0};
       bool outside = false;
       cell_of<D>(T, pn, cn, outside);
       A.curkey[i] = key_of(flat_cell<D>(T, cn), false);
     }
-    store_list_record<D>(A.pos_out, A.dat_out, i, T, pn, fluid_record<D>(S.phys, T, vn, rn, A.n_walls > 0));
+    const auto rec = fluid_record<D>(S.phys, T, vn, rn, A.n_walls > 0);
+    if constexpr (F == TG_FP32C) {
+      if (A.carry) {
+        A.travel_out[i] = far * 1.00001f;
+        R v2 = R(0), a2 = R(0);
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+          A.next.vel[k][i] = vn[k];
+          v2 += vn[k] * vn[k];
+          a2 += dv[k] * dv[k];
+        }
+        A.next.rho[i] = rn;
+        fold_time_step(A.dt_next, tk, time_step(S.phys, T, sqrtf(v2), sqrtf(a2), rn, rec.c));
+      }
+    }
+    store_list_record<D>(A.pos_out, A.dat_out, i, T, pn, rec);
     return;
   }
   int c[3] = {0, 0, 0};
