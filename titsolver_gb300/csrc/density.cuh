@@ -204,15 +204,6 @@ __global__ void __launch_bounds__(kDensityBlock) k_density64(CloudArgs<D> A) {
   if (A.hashes != nullptr) A.hashes[id] = hs;
 }
 
-// sqrt(x) for x >= 0 from the hardware's approximate square root (relative
-// error below 2^-22): the values of a hundred neighbours are summed, so their
-// rounding does not reach the sum's.
-__device__ __forceinline__ float sqrt_approx(float x) {
-  float y;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // FP32 form, one thread per point: the walk over the candidates bounds it
 // (about a thousand per point in the clusters, 75% of the issue slots).  The
 // predicate is the reference's on the rounded positions, uncontracted; the

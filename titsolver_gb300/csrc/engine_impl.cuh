@@ -136,7 +136,7 @@ class Engine final : public EngineBase {
       double most = 0.0;
       for (size_t t = 0; t < C.tanks.size(); ++t) {
         const TankDev& T = C.tankdev[t];
-        const double R = (F == TG_FP32C ? 1.1 : 1.06) * T.R_f;
+        const double R = 1.1 * T.R_f;
         const double ball = D == 2 ? 3.14159265358979 * R * R : 4.18879020478639 * R * R * R;
         most = std::max(most, ball * T.rho0 / T.m);
         // Tank-local FP32 coordinates must resolve the radius.
@@ -164,7 +164,8 @@ class Engine final : public EngineBase {
         e = C.alloc(reinterpret_cast<void**>(&datrec_b_), sizeof(DatRec) * (C.n + kListScan));
         if (e == cudaSuccess && F == TG_FP64) {
           e = C.alloc(reinterpret_cast<void**>(&posrec_b_), sizeof(PosRec) * C.n);
-        } else if (e == cudaSuccess) {
+        }
+        if (e == cudaSuccess) {
           e = C.alloc(reinterpret_cast<void**>(&travel_), sizeof(float) * C.n);
         }
       }
@@ -179,9 +180,9 @@ class Engine final : public EngineBase {
   }
 
   int chain(const Context& C) const override {
-    // Not where the lists would serve the FP64 pipe, which pays for every
-    // entry, nor after a step of this context had to be repeated.
-    return F == TG_FP32C && C.lists && C.list_redos == 0 &&
+    // Not where the FP64 pipe would pay for every further entry, nor after a
+    // step of this context had to be repeated.
+    return (F == TG_FP32C || list_team(C) > 1) && C.lists && C.list_redos == 0 &&
                    C.P.post_integrate != TG_POST_SHIFTING && !C.faces.on
                ? kListChain
                : 1;
@@ -381,6 +382,7 @@ class Engine final : public EngineBase {
     a.carry = 0;
     a.mode = kPassRK;
     a.walls_keep = 0;
+    a.walls = C.n_wall > 0 ? 1 : 0;
     a.stop = C.d_err + 1;
     return a;
   }
@@ -601,10 +603,15 @@ class Engine final : public EngineBase {
     C.launches += 1;
   }
   void launch_list_walls(Context& C, const ListArgs<D, F>& A) {
+    const int team = list_team(C) > 1 ? 8 : 4;
     const int64_t cap = 16 * static_cast<int64_t>(C.sm_count > 0 ? C.sm_count : 152);
     const unsigned grid =
-        static_cast<unsigned>(std::min<int64_t>(grid_for(C.n_wall * kListWallTeam, 128), cap));
-    k_list_walls<D, F, K><<<grid, 128, 0, C.stream>>>(A);
+        static_cast<unsigned>(std::min<int64_t>(grid_for(C.n_wall * team, 128), cap));
+    if (team == 8) {
+      k_list_walls<D, F, K, 8><<<grid, 128, 0, C.stream>>>(A);
+    } else {
+      k_list_walls<D, F, K, 4><<<grid, 128, 0, C.stream>>>(A);
+    }
     C.launches += 1;
   }
   template<int Phys>

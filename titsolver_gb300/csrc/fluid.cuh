@@ -152,6 +152,7 @@ struct StageArgs {
   int carry;         // gather every field into Y (prepare and split passes)
   int mode;          // update rule of the force pass (kPass*)
   int walls_keep;    // k_walls: keep the carried wall densities
+  int walls;         // the wall pass follows
   unsigned* fbox;     // per-tank fluid bounding box (k_reorder)
   FaceArgs fc;        // boundary faces (fc.on = 0: particle walls)
   const uint32_t* stop;  // not zero: a step on neighbour lists has to be
@@ -590,6 +591,29 @@ __device__ __forceinline__ bool finite_bits(double x) {
           0x7ff0000000000000ull) != 0x7ff0000000000000ull;
 }
 
+// Cell and FP32 offset from its corner of an FP64 position, from its fixed
+// point in 2^-28 cells (2 FP64 operations per axis instead of 10): cell_of's
+// cells up to that unit's rounding.  Positions beyond the fixed point's range
+// or the grid go by cell_of.
+template<int D>
+__device__ __forceinline__ void cell_and_offset(const TankDev& T, const double* p, int* c,
+                                                float* o, bool& outside) {
+  bool in = true;
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    // 2^52 + 2^51 + the integer: in range while the sum stays in [2^52, 2^53).
+    const double t = fma(p[k] - T.lo[k], T.list_inv_unit, 6755399441055744.0);
+    const long long q = __double_as_longlong(t) - 0x4338000000000000ll;
+    const long long cell = q >> 28;
+    in = in && (__double2hiint(t) >> 20) == 0x433 && cell >= 0 && cell < T.nc[k];
+    c[k] = static_cast<int>(cell);
+    o[k] = static_cast<float>(static_cast<int>(q & 0xfffffffll)) * T.list_unit_f;
+  }
+  if (in) return;
+  cell_of<D>(T, p, c, outside);
+  cell_offset<D>(T, c, p, o);
+}
+
 // ---------------------------------------------------------------------------
 // Cell key (and FP32 offset) of every home particle from its FP64 position;
 // runs after an upload.  The tank comes from the upload index.
@@ -603,14 +627,13 @@ __global__ void __launch_bounds__(256)
   const TankDev& T = tanks[tank_of[X.id[i] & kIdMask]];
   double p[3] = {X.pos[0][i], X.pos[1][i], D == 3 ? X.pos[2][i] : 0.0};
   int c[3] = {0, 0, 0};
+  float o[3] = {0.f, 0.f, 0.f};
   bool outside = false;
-  cell_of<D>(T, p, c, outside);
+  cell_and_offset<D>(T, p, c, o, outside);
   X.key[i] = key_of(flat_cell<D>(T, c), (X.id[i] & kWallBit) != 0);
   if constexpr (F == TG_FP32C) {
 #pragma unroll
-    for (int k = 0; k < D; ++k) {
-      X.off[k][i] = static_cast<float>(p[k] - (T.lo[k] + c[k] * T.cs));
-    }
+    for (int k = 0; k < D; ++k) X.off[k][i] = o[k];
   }
   if (outside) {
     bool finite = true;
@@ -775,8 +798,11 @@ __global__ void __launch_bounds__(256) k_reorder(StageArgs<D, F> A) {
         double pr, c;
         tait_f64(A.phys, T, rho, pr, c);
         const double inv = 1.0 / rho;
+        // With walls, the pad word takes the potential for the wall pass.
+        const double H =
+            A.walls && !A.walls_keep ? potential_f64(A.phys, T, rho) : 0.0;
         A.datrec[j] = Dat64{v[0], v[1], D == 3 ? v[2] : 0.0, rho,
-                            pr * inv * inv, c, inv, 0.0};
+                            pr * inv * inv, c, inv, H};
         if (A.compute_dt) {
           double dvv[3];
 #pragma unroll
@@ -937,12 +963,11 @@ __global__ void __launch_bounds__(128)
           const double s2 = dist2_exact<D>(pb, pe, d);
           if (s2 > R2) continue;
           const Dat64 b = load_dat(A.datrec, j);
-          const double W = w * KernelPoly<K>::value(sqrt(s2) * hinv);
-          const double Vb = m * b.invrho;
-          double Hb = potential_f64(A.phys, T, b.rho);
+          const double VW = b.invrho * KernelPoly<K>::value(sqrt_f64(s2) * hinv);
+          double Hb = b.pad;
           if (A.fc.on) Hb += A.phys.g * dot_d<D>(d, ne) * ne[1];
-          S += Vb * W;
-          H += Vb * Hb * W;
+          S += VW;
+          H = fma(VW, Hb, H);
         }
       };
       float oc[3] = {0.f, 0.f, 0.f};
@@ -954,8 +979,8 @@ __global__ void __launch_bounds__(128)
         H += __shfl_xor_sync(tmask, H, o, kWallTeam);
       }
       if (tl == 0) {
-        const double Hs = fabs(S) <= 6.0554544523933395e-06 ? 0.0 : H / S;
-        const double rho_e = density_from_potential_f64(A.phys, T, Hs);
+        const double Hs = fabs(S * (w * m)) <= 6.0554544523933395e-06 ? 0.0 : H / S;
+        const double rho_e = wall_density_f64(A.phys, T, Hs);
         double pr, cc;
         tait_f64(A.phys, T, rho_e, pr, cc);
         const double inv = 1.0 / rho_e;

@@ -20,8 +20,9 @@
 // repeats the step with a sort per stage (tg_step).  Nothing is approximated:
 // the predicate |r_ab| <= R is applied to every entry in every stage.
 //
-// Chains.  The compensated form's steps within one tg_step call share the
-// lists (kListChain at a time): the lists are as much wider, and the first
+// Chains.  The steps within one tg_step call share the lists (kListChain at
+// a time; in the plain form only those of small runs, whose sorts and builds
+// are chains of short launches): the lists are as much wider, and the first
 // step's last stage hands its state on in the records.  The home state
 // is written by the chain's last step, so a stop repeats the whole chain.
 //
@@ -173,7 +174,7 @@ __device__ __forceinline__ void store_list_record(const int4*, Dat32* dat, int64
 }
 
 // FluidEquations::compute_time_step (fluid_equations.hpp:205-230) of one
-// particle, compensated form.
+// particle, in either form (rho: the density, or its deviation).
 __device__ __forceinline__ float time_step(const PhysDev& P, const TankDev& T, float speed,
                                            float accel, float drho, float c) {
   const float h = T.h_f;
@@ -181,6 +182,15 @@ __device__ __forceinline__ float time_step(const PhysDev& P, const TankDev& T, f
   const float dt_vi = P.c_visc_f * h * h * (T.rho0_f + drho) / P.mu_f;
   const float dt_fo = P.c_force_f * sqrtf(h / fmaxf(accel, P.g_f));
   return fminf(dt_ac, fminf(dt_vi, dt_fo));
+}
+
+__device__ __forceinline__ double time_step(const PhysDev& P, const TankDev& T, double speed,
+                                            double accel, double rho, double c) {
+  const double h = T.h;
+  const double dt_ac = P.cfl * h / (c + speed);
+  const double dt_vi = P.c_visc * h * h * rho / P.mu;
+  const double dt_fo = P.c_force * sqrt(h / fmax(accel, P.g));
+  return fmin(dt_ac, fmin(dt_vi, dt_fo));
 }
 
 // Minimum over a tank, from the lanes that are here: one atomic for those of
@@ -194,6 +204,10 @@ __device__ __forceinline__ void fold_time_step(double* dt, uint32_t tk, float mi
   if (same && static_cast<int>(threadIdx.x & 31u) != __ffs(here) - 1) return;
   const double d = static_cast<double>(__uint_as_float(bits));
   if (d < *static_cast<volatile double*>(dt + tk)) atomic_min_pos(dt + tk, d);
+}
+
+__device__ __forceinline__ void fold_time_step(double* dt, uint32_t tk, double mine) {
+  if (mine < *static_cast<volatile double*>(dt + tk)) atomic_min_pos(dt + tk, mine);
 }
 
 // ---------------------------------------------------------------------------
@@ -247,19 +261,10 @@ __global__ void __launch_bounds__(256) k_list_gather(ListArgs<D, F> A) {
         a2 += a * a;
         v2 += v[k] * v[k];
       }
-      // FluidEquations::compute_time_step (fluid_equations.hpp:205-230).
-      if constexpr (F == TG_FP64) {
-        const double h = T.h, speed = sqrt(v2);
-        const double dt_ac = S.phys.cfl * h / (rec.c + speed);
-        const double dt_vi = S.phys.c_visc * h * h * rho / S.phys.mu;
-        const double dt_fo = S.phys.c_force * sqrt(h / fmax(sqrt(a2), S.phys.g));
-        dt_a = fmin(dt_ac, fmin(dt_vi, dt_fo));
-        v_a = __double2float_ru(speed);
-      } else {
-        const float speed = sqrtf(v2);
-        dt_a = static_cast<double>(time_step(S.phys, T, speed, sqrtf(a2), rho, rec.c));
-        v_a = speed;
-      }
+      const R speed = sqrt(v2);
+      dt_a = static_cast<double>(time_step(S.phys, T, speed, sqrt(a2), rho, rec.c));
+      if constexpr (F == TG_FP64) v_a = __double2float_ru(speed);
+      else v_a = speed;
     }
     store_list_record<D>(A.pos_in, A.dat_in, j, T, p, rec);
   }
@@ -609,35 +614,6 @@ __device__ __forceinline__ T list_g(T t, T q, T rinv) {
   }
 }
 
-__device__ __forceinline__ float rsqrt_seed(float x) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ double rsqrt_seed(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  return y;
-}
-__device__ __forceinline__ double rcp_seed(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  return y;
-}
-
-// 1 / x and sqrt(x), from the hardware seeds by one third-order iteration.
-__device__ __forceinline__ double rcp_f64(double x) {
-  const double y = rcp_seed(x);
-  const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
-__device__ __forceinline__ double sqrt_f64(double x) {
-  const double y = rsqrt_seed(x);
-  const double r = x * y;
-  const double e = fma(-r, y, 1.0);
-  return __double2hiint(x) == 0 ? 0.0 : fma(r, e * fma(e, 0.375, 0.5), r);
-}
-
 __device__ __forceinline__ Dat32 load_dat_wide(const Dat32* p, uint32_t j) {
   Dat32 r;
   asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -645,12 +621,6 @@ __device__ __forceinline__ Dat32 load_dat_wide(const Dat32* p, uint32_t j) {
         "=f"(r.pad)
       : "l"(p + j));
   return r;
-}
-
-__device__ __forceinline__ float rcp_approx(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
 }
 
 // Compensated form, one target.
@@ -860,26 +830,13 @@ struct ListPairF64 {
 };
 
 // ---------------------------------------------------------------------------
-// rho(H) of the Tait law with xi = 7, rho0 u^(1/6) with u = 1 + 6 H / cs0^2:
-// the FP32 power y0 (relative error below 2^-19) times the binomial series
-// of (u / y0^6)^(1/6) to second order (truncation below 2^-57), 14 FP64
-// operations in a chain instead of pow's.
-__device__ __forceinline__ double wall_density_f64(const PhysDev& P, const TankDev& T, double H) {
-  if (!P.xi_is_7 || P.eos != TG_EOS_TAIT) return density_from_potential_f64(P, T, H);
-  const double u = 1.0 + 6.0 * H / (T.cs0 * T.cs0);
-  // FP32's range with room for its powers (false for a NaN as well).
-  if (!(u > 1e-30 && u < 1e30)) return density_from_potential_f64(P, T, H);
-  const double y0 = static_cast<double>(powf(static_cast<float>(u), 1.f / 6.f));
-  const double y2 = y0 * y0, y6 = y2 * y2 * y2;
-  const double e = (u - y6) * rcp_f64(y6);
-  return T.rho0 * fma(y0, e * fma(e, -5.0 / 72.0, 1.0 / 6.0), y0);
-}
-
-// Wall extrapolation (k_walls) over the walls' lists: teams of 8 lanes take
-// the listed walls in turn, the lanes the list's groups of four entries.
-constexpr int kListWallTeam = 8;
-
-template<int D, int F, int K>
+// Wall extrapolation (k_walls) over the walls' lists: teams of lanes take the
+// listed walls in turn, the lanes the list's groups of four entries.  Four
+// lanes, eight for the small runs whose passes are chains of latencies
+// (measured in ms per step for 8 / 4 / 2 lanes: 24 3D tanks .163 / .129 /
+// .131, 3D 2M .121 / .101 / .097, plain 3D 250k .366 / .297 / .297, 2D 1.28M
+// .037 / .039 / .050; 800 particles with shifting 297 / 310 us per step).
+template<int D, int F, int K, int Team>
 __global__ void __launch_bounds__(128) k_list_walls(ListArgs<D, F> A) {
   if (*A.stop != 0u) return;
   const StageArgs<D, F>& S = A.S;
@@ -887,10 +844,10 @@ __global__ void __launch_bounds__(128) k_list_walls(ListArgs<D, F> A) {
   const bool all = S.fbox == nullptr;
   const uint32_t* list = all ? S.wall_list : S.wall_active;
   const int64_t count = all ? S.wall_count[0] : S.wall_count[1];
-  const int tl = static_cast<int>(threadIdx.x % kListWallTeam);
-  const unsigned tmask = team_mask<kListWallTeam>();
-  const int64_t teams = static_cast<int64_t>(gridDim.x) * blockDim.x / kListWallTeam;
-  for (int64_t w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / kListWallTeam;
+  const int tl = static_cast<int>(threadIdx.x % Team);
+  const unsigned tmask = team_mask<Team>();
+  const int64_t teams = static_cast<int64_t>(gridDim.x) * blockDim.x / Team;
+  for (int64_t w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / Team;
        w < count; w += teams) {
     const uint32_t ew = list[w];
     const TankDev& T = S.tanks[tank_of_key(S.skey[ew], S.tank_off, S.ntanks)];
@@ -902,7 +859,7 @@ __global__ void __launch_bounds__(128) k_list_walls(ListArgs<D, F> A) {
       double pe[3] = {0.0, 0.0, 0.0};
       load_pos(A.pos_in, ew, pe);
       double Ss = 0.0, H = 0.0;
-      for (uint32_t p = 4 * tl; p < m; p += 4 * kListWallTeam) {
+      for (uint32_t p = 4 * tl; p < m; p += 4 * Team) {
         const uint4 g = groups[(p >> 2) * 32];
         const uint32_t js[4] = {g.x, g.y, g.z, g.w};
         for (uint32_t q = 0; q < 4u && p + q < m; ++q) {
@@ -919,9 +876,9 @@ __global__ void __launch_bounds__(128) k_list_walls(ListArgs<D, F> A) {
         }
       }
 #pragma unroll
-      for (int o = kListWallTeam / 2; o > 0; o >>= 1) {
-        Ss += __shfl_xor_sync(tmask, Ss, o, kListWallTeam);
-        H += __shfl_xor_sync(tmask, H, o, kListWallTeam);
+      for (int o = Team / 2; o > 0; o >>= 1) {
+        Ss += __shfl_xor_sync(tmask, Ss, o, Team);
+        H += __shfl_xor_sync(tmask, H, o, Team);
       }
       if (tl == 0) {
         const double Hs = fabs(Ss * (T.m * T.w)) <= 6.0554544523933395e-06 ? 0.0 : H / Ss;
@@ -933,7 +890,7 @@ __global__ void __launch_bounds__(128) k_list_walls(ListArgs<D, F> A) {
       const Dat32 e = A.dat_in[ew];
       get_coords<D>(e, own.x);
       Kahan Ss, H;
-      for (uint32_t p = 4 * tl; p < m; p += 4 * kListWallTeam) {
+      for (uint32_t p = 4 * tl; p < m; p += 4 * Team) {
         const uint4 g = groups[(p >> 2) * 32];
         const uint32_t js[4] = {g.x, g.y, g.z, g.w};
         for (uint32_t q = 0; q < 4u && p + q < m; ++q) {
@@ -942,8 +899,8 @@ __global__ void __launch_bounds__(128) k_list_walls(ListArgs<D, F> A) {
           const float s2 = own.rab(b, d);
           if (s2 > T.list_hi_f) continue;
           if (s2 >= T.list_lo_f && !within_fp64<D>(A.pin, ew, js[q], T.radius2)) continue;
-          const float W = T.w_f * KernelPoly<K>::value(sqrtf(s2) * hq);
-          const float ib = D == 2 ? b.invrho : __frcp_rn(T.rho0_f + b.drho);
+          const float W = T.w_f * KernelPoly<K>::value(sqrt_approx(s2) * hq);
+          const float ib = D == 2 ? b.invrho : rcp_approx(T.rho0_f + b.drho);
           const float Vb = T.m_f * ib;
           float Hb = potential_f32(S.phys, T, b.drho);
           if (S.fc.on) {
@@ -958,9 +915,9 @@ __global__ void __launch_bounds__(128) k_list_walls(ListArgs<D, F> A) {
       }
       float Sv = Ss.value(), Hv = H.value();
 #pragma unroll
-      for (int o = kListWallTeam / 2; o > 0; o >>= 1) {
-        Sv += __shfl_xor_sync(tmask, Sv, o, kListWallTeam);
-        Hv += __shfl_xor_sync(tmask, Hv, o, kListWallTeam);
+      for (int o = Team / 2; o > 0; o >>= 1) {
+        Sv += __shfl_xor_sync(tmask, Sv, o, Team);
+        Hv += __shfl_xor_sync(tmask, Hv, o, Team);
       }
       if (tl == 0) {
         const float Hs = fabsf(Sv) <= 6.0554544523933395e-06f ? 0.f : Hv / Sv;
@@ -1088,19 +1045,17 @@ __device__ __forceinline__ void list_epilogue(const ListArgs<D, F>& A, int64_t i
       A.curkey[i] = key_of(flat_cell<D>(T, cn), false);
     }
     const auto rec = fluid_record<D>(S.phys, T, vn, rn, A.n_walls > 0);
-    if constexpr (F == TG_FP32C) {
-      if (A.carry) {
-        A.travel_out[i] = far * 1.00001f;
-        R v2 = R(0), a2 = R(0);
+    if (A.carry) {
+      A.travel_out[i] = far * 1.00001f;
+      R v2 = R(0), a2 = R(0);
 #pragma unroll
-        for (int k = 0; k < D; ++k) {
-          A.next.vel[k][i] = vn[k];
-          v2 += vn[k] * vn[k];
-          a2 += dv[k] * dv[k];
-        }
-        A.next.rho[i] = rn;
-        fold_time_step(A.dt_next, tk, time_step(S.phys, T, sqrtf(v2), sqrtf(a2), rn, rec.c));
+      for (int k = 0; k < D; ++k) {
+        A.next.vel[k][i] = vn[k];
+        v2 += vn[k] * vn[k];
+        a2 += dv[k] * dv[k];
       }
+      A.next.rho[i] = rn;
+      fold_time_step(A.dt_next, tk, time_step(S.phys, T, sqrt(v2), sqrt(a2), rn, rec.c));
     }
     store_list_record<D>(A.pos_out, A.dat_out, i, T, pn, rec);
     return;
