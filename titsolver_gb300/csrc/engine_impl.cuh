@@ -617,8 +617,10 @@ class Engine final : public EngineBase {
   template<int Phys>
   void launch_list_forces(Context& C, const ListArgs<D, F>& A, int team) {
     const int block = std::min(C.force_block, 128);
-    const size_t smem =
-        F == TG_FP32C ? sizeof(uint32_t) * kBandCap * static_cast<size_t>(block) : 0;
+    // The band lists of the compensated B-spline sums.
+    const size_t smem = F == TG_FP32C && !KernelPoly<K>::deriv_over_q
+                            ? sizeof(uint32_t) * kBandCap * static_cast<size_t>(block)
+                            : 0;
     const unsigned grid = grid_for(C.n * team, block);
     if (team == 16) {
       k_list_forces<D, F, K, Phys, 16><<<grid, block, smem, C.stream>>>(A);

@@ -1066,18 +1066,22 @@ __device__ __forceinline__ void list_epilogue(const ListArgs<D, F>& A, int64_t i
 }
 
 // Launch bounds (128-thread blocks per SM) and records in flight per lane of
-// the pair loop.  FP64: its pipe is the limit.  Compensated, measured for the
-// three passes of a step at 2M (3D) / 1.28M (2D) fluid particles in ms: 3D
-// 7 blocks, 2 records 1.62 (5 / 4: 1.68, 6 / 4: 1.85, 8 / 1: 1.64, 8 / 2:
-// 1.92, spills); 2D 8 blocks, 2 records 0.611 (6 / 4: 0.635, 8 / 1: 0.631).
+// the pair loop.  FP64: its pipe is the limit.  Compensated: the gathers take
+// two thirds of L1's wavefronts and the pairs three fifths of the issue slots
+// at the same time.  Measured for the three passes of a step (in a chain of
+// two) at 2M (3D) / 1.28M (2D) fluid particles in ms, blocks x records: 3D
+// 7 x 2 1.59, 6 x 4 1.585, 8 x 2 1.62, 6 x 2 1.62, 9 x 2 1.75, 5 x 4 1.69,
+// 8 x 1 1.68; 2D 9 x 2 .631, 8 x 2 .642, 10 x 2 .665, 7 x 2 .656, 8 x 4 .638,
+// 10 x 1 .636.  With a predicate per entry and a check of the list's end: 3D
+// 1.69, 2D .631.
 template<int D, int F>
 constexpr int list_min_blocks() {
-  return F == TG_FP64 ? 4 : D == 3 ? 7 : 8;
+  return F == TG_FP64 ? 4 : D == 3 ? 7 : 9;
 }
 constexpr uint32_t kListBatch = 2;
 
 // Team lanes per target take the list's groups of four entries in turn.
-// The compensated sums take one add per group (2D) or two groups (3D).
+// The compensated sums take one add per two groups.
 template<int D, int F, int K, int Phys, int Team>
 __global__ void __launch_bounds__(128, list_min_blocks<D, F>()) k_list_forces(ListArgs<D, F> A) {
   using R = typename StageArgs<D, F>::R;
@@ -1133,45 +1137,56 @@ __global__ void __launch_bounds__(128, list_min_blocks<D, F>()) k_list_forces(Li
   } else {
     ListPairF32<D, F, K, Phys> acc;
     acc.init(A, T, i);
+    // B-splines: entries in the band around R^2 wait for the FP64 predicate
+    // until the list is done (kBandCap of them; more take a second pass).
+    // Wendland kernels need no predicate: beyond R their t is cut to 0, and
+    // in the band t <= 2^-15 makes g at most t^3 = 2^-45 of its peak, below
+    // the rounding of every sum it could enter.
+    constexpr bool kBand = !KernelPoly<K>::deriv_over_q;
     const float lo = T.list_lo_f, hi = T.list_hi_f;
-    // Entries in the band around R^2 wait for the FP64 predicate until the
-    // list is done (kBandCap of them; more take a second pass).
     extern __shared__ uint32_t s_band[];
     uint32_t* slots = s_band + threadIdx.x;
     uint32_t nb = 0;
+    const auto pair = [&](const Dat32& b, uint32_t j) {
+      float d[3];
+      float s2 = acc.rab(b, d);
+      if constexpr (kBand) {
+        if (s2 >= lo && s2 <= hi) {
+          if (nb < static_cast<uint32_t>(kBandCap)) slots[nb * blockDim.x] = j;
+          ++nb;
+        }
+        // Entries beyond the radius add zero (the kernel vanishes at twice
+        // the radius): no branch between the pairs.
+        if (!(s2 < lo)) s2 = 4.f * hi;
+      }
+      acc.add(A, T, d, s2, b);
+    };
     acc.open();
-    uint4 g = m > 4u * tl ? groups[tl * 32] : make_uint4(0u, 0u, 0u, 0u);
-    for (uint32_t p = 4 * tl; p < m; p += 4 * Team) {
+    uint32_t p = 4 * tl, done = 0;
+    uint4 g = p < m ? groups[tl * 32] : make_uint4(0u, 0u, 0u, 0u);
+    for (; p + 4u <= m; p += 4 * Team) {
       const uint32_t js[4] = {g.x, g.y, g.z, g.w};
       if (p + 4u * Team < m) g = groups[((p >> 2) + Team) * 32];  // the next entries
 #pragma unroll
       for (uint32_t q0 = 0; q0 < 4u; q0 += kListBatch) {
         Dat32 b[kListBatch];
 #pragma unroll
-        for (uint32_t q = 0; q < kListBatch; ++q) {
-          b[q] = load_dat_wide(A.dat_in, p + q0 + q < m ? js[q0 + q] : static_cast<uint32_t>(i));
-        }
+        for (uint32_t q = 0; q < kListBatch; ++q) b[q] = load_dat_wide(A.dat_in, js[q0 + q]);
 #pragma unroll
-        for (uint32_t q = 0; q < kListBatch; ++q) {
-          float d[3];
-          const float s2 = acc.rab(b[q], d);
-          const bool valid = p + q0 + q < m;
-          if (valid && s2 >= lo && s2 <= hi) {
-            if (nb < static_cast<uint32_t>(kBandCap)) slots[nb * blockDim.x] = js[q0 + q];
-            ++nb;
-          }
-          // Entries beyond the radius add zero (the kernel vanishes at twice
-          // the radius): no branch between the pairs.
-          acc.add(A, T, d, valid && s2 < lo ? s2 : 4.f * hi, b[q]);
-        }
+        for (uint32_t q = 0; q < kListBatch; ++q) pair(b[q], js[q0 + q]);
       }
-      if (D == 2 || (p & 4u) != 0u) {
+      if ((++done & 1u) == 0u) {
         acc.close();
         acc.open();
       }
     }
+    if (p < m) {  // the last group, up to three entries
+      pair(load_dat_wide(A.dat_in, g.x), g.x);
+      if (p + 1u < m) pair(load_dat_wide(A.dat_in, g.y), g.y);
+      if (p + 2u < m) pair(load_dat_wide(A.dat_in, g.z), g.z);
+    }
     acc.close();
-    if (nb != 0u) {
+    if (kBand && nb != 0u) {
       const auto decide = [&](uint32_t j) {
         const Dat32 b = load_dat_wide(A.dat_in, j);
         float d[3];
