@@ -236,10 +236,16 @@ __device__ __forceinline__ T face_unit_segment(T eta, T zmin, T zmax, unsigned s
       total += face_primitive<K, I, Anti, T>(eta, hi) - face_primitive<K, I, Anti, T>(eta, lo);
       return;
     }
-    // The clipped ends (a segment outside the circle gives P(+-zc) twice,
-    // i.e. zero, as the early return above does).
-    if (!(skip & 2u)) total += face_primitive<K, I, Anti, T>(eta, M::min(M::max(zmax, -zc), zc));
-    if (!(skip & 1u)) total -= face_primitive<K, I, Anti, T>(eta, M::min(M::max(zmin, -zc), zc));
+    // The one clipped end that is left, whichever it is, so that the lanes of
+    // a group evaluate the primitive together, a lower end in one and an
+    // upper end in the next (a chain of segments outside the circle gives
+    // P(+-zc) at both its ends, i.e. zero, as the early return above does).
+    // 2D pool of 12,800 fluid, 4 steps with shifting: 3954 -> 3600 us.
+    if (skip == 3u) return;
+    const bool upper = (skip & 1u) != 0u;
+    const T z = M::min(M::max(upper ? zmax : zmin, -zc), zc);
+    const T v = face_primitive<K, I, Anti, T>(eta, z);
+    total += upper ? v : -v;
   });
   return total;
 }
