@@ -145,20 +145,22 @@ typedef struct tg_params {
   int32_t cells_per_radius; /* grid cells per support radius, 1..3 */
   int32_t kahan;            /* FP32C: 1 = compensated sums, 0 = plain */
   int32_t device;           /* CUDA device ordinal; -1 = the current one */
-  int32_t staging;          /* 2D FP32C: copy each block's neighbour
-                               window into shared memory with bulk copies
-                               (1) or read it through L1 (0, default;
-                               measured faster on GB300) */
+  int32_t staging;          /* 2D FP32C, in the force passes that walk
+                               cells (see tg_step): copy each block's
+                               neighbour window into shared memory with
+                               bulk copies (1) or read it through L1 (0,
+                               default; measured faster on GB300) */
   int32_t eos;              /* TG_EOS_TAIT (default) | TG_EOS_LINEAR_TAIT */
   int32_t face_fp32;        /* TG_FP32C with face walls: the closed-form face
                                integrals in FP32 (1) or FP64 (0, default).
                                FP32 runs the face passes ~1.7x faster in 3D
                                at a larger drift from the FP64 form; must be
                                0 with TG_FP64. */
-  int32_t resort;           /* 1 (default): between stages, re-sort only the
-                               particles whose cell changed and merge them
-                               into the previous order; 0: a full radix sort
-                               every stage.  Same order either way. */
+  int32_t resort;           /* 1 (default): from one sort to the next,
+                               re-sort only the particles whose cell changed
+                               and merge them into the previous order; 0: a
+                               full radix sort each time.  Same order either
+                               way. */
   double xi;      /* Tait polytropic index */
   double g;       /* gravity, acting along -axis 1 */
   double mu;      /* Morris dynamic viscosity */
@@ -181,7 +183,7 @@ typedef struct tg_tank {
 
 /* Accumulated device time per kernel group, in milliseconds. */
 typedef struct tg_profile {
-  double sort_ms;    /* cell keys, radix sort, cell table */
+  double sort_ms;    /* cell keys, radix sort, cell table, neighbour lists */
   double reorder_ms; /* gather into cell order, dt reduction */
   double walls_ms;   /* wall state extrapolation */
   double forces_ms;  /* fused continuity + momentum + RK update */
@@ -223,7 +225,12 @@ int tg_particles_update(tg_context* ctx, const double* r, const double* v,
 int tg_prepare(tg_context* ctx);
 
 /* Advance every tank by n_steps integrator steps (each with its own dt).
- * dt_out (n_tanks doubles, may be NULL) receives the last step's dt. */
+ * dt_out (n_tanks doubles, may be NULL) receives the last step's dt.
+ * SSPRK3 and SSPRK2 steps run on neighbour lists that hold for one step, or
+ * for two steps of one call.  Steps whose particles leave the lists' reach
+ * or overflow them are repeated with a sort and a cell walk per stage, which
+ * the other integrators, and particle sets whose lists would take more than
+ * a third of the free device memory, use throughout. */
 int tg_step(tg_context* ctx, int32_t n_steps, double* dt_out);
 
 /* Per-tank accumulated time (n_tanks doubles). */
@@ -351,10 +358,11 @@ int tg_tank_faces(tg_context* ctx, int32_t tank, int32_t n_faces,
 /* ---- launch shape and the autotuner ----------------------------------- */
 /* Launch shape of a context: the grid's cell size (cells_per_radius cells
  * across the kernel support radius, as GridSearch{spacing} picks the cell
- * size in source/tit/geom/search/grid_search.hpp:73-113), the force pass's
- * threads per block, and its lanes per fluid particle (1, 2 or 4: the lanes
- * split the particle's neighbour cells, so a warp advances 32, 16 or 8
- * particles; 2 and 4 exist for the Wendland C2 and C4 kernels). */
+ * size in source/tit/geom/search/grid_search.hpp:73-113), and, for force
+ * passes that walk cells, the threads per block and the lanes per fluid
+ * particle (1, 2 or 4: the lanes split the particle's neighbour cells, so a
+ * warp advances 32, 16 or 8 particles; 2 and 4 exist for the Wendland C2 and
+ * C4 kernels).  Force passes on neighbour lists choose their own. */
 typedef struct tg_tuning {
   int32_t cells_per_radius;   /* 1..3 */
   int32_t block_size;         /* 64, 128 or 256 */

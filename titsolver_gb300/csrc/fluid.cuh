@@ -13,9 +13,13 @@
 //               update, SSPRK linear combination, and the cell key (and
 //               FP32 cell offset) of the new position for the next sort
 //               (fluid_equations.hpp:232-305, time_integrator.hpp:203-223)
-// Keys come from FP64 positions in k_keys only after an upload; afterwards
-// k_forces and k_walls write them, so no kernel recomputes cells from FP64
-// positions (FP64 issue is scarce on GB300).
+// The last pass over the particles writes their keys by fixed-point
+// arithmetic (cell_and_offset); k_keys computes them from FP64 positions only
+// after an upload or update (FP64 issue is scarce on GB300).
+// SSPRK steps run these stages only where the neighbour lists of
+// pairlist.cuh do not serve: steps that the lists' bounds stop, and sets
+// whose lists would take too much memory.  The other integrators, and the
+// prepare passes outside a step, always run them.
 #pragma once
 
 #include <cstdint>

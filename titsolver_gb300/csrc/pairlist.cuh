@@ -18,7 +18,10 @@
 // delta, or a list past its capacity, raises *stop.  The last stage and all
 // later kernels then leave the home state as the step found it, and the host
 // repeats the step with a sort per stage (tg_step).  Nothing is approximated:
-// the predicate |r_ab| <= R is applied to every entry in every stage.
+// every entry's |r_ab| is taken anew in every stage, and an entry beyond R
+// adds nothing: by the predicate |r_ab| <= R, or, in the compensated form
+// with a Wendland kernel, by the kernel itself, whose clamped factor
+// max(1 - |r_ab| / R, 0) makes each of its terms an exact zero there.
 //
 // Chains.  The steps within one tg_step call share the lists (kListChain at
 // a time; in the plain form only those of small runs, whose sorts and builds
