@@ -23,7 +23,7 @@ neighbour rebuilds, three fused force passes).
 * ``e2e``: the same metric through the C ABI with host buffers: every step
   uploads r, v, rho, dv/dt from pinned host memory, steps, and downloads
   them again (tg_particles_update / tg_step / tg_particles_download_state).
-* ``roofline``: the fused force kernel (k_forces): algorithmic bytes per
+* ``roofline``: the fused force kernel (k_list_forces): algorithmic bytes per
   launch = fluid particles x 3S (S = state bytes per particle) over its mean
   launch time from a profiled pass with CUDA events on the same stream.
   The kernel is not HBM-bound; ``compute`` gives its FP32 work per launch
@@ -216,15 +216,16 @@ def forces_traffic_source(dim: int, form: str) -> str | None:
 
 
 # FP32 floating-point operations of the compensated force pass, counted from
-# the kernel source (fluid.cuh, PairF32::add with the textbook terms:
+# the kernel source (pairlist.cuh, ListPairF32::add with the textbook terms:
 # Wendland C2, delta-SPH diffusion, Monaghan viscosity; an FMA counts 2, a
-# reciprocal square root or reciprocal 1).  Per accepted pair: rsqrt 1,
-# r and q 2, kernel gradient factor 6, v_ab . r_ab 3d - 1, density
-# difference 1, diffusion 3, continuity term 2, Monaghan term 9, momentum
-# coefficient 4, sums 1 + 2d.  Per candidate: r_ab d (plus the 3D row
-# shift 2) and |r_ab|^2 2d - 1.
-FLOPS_PER_PAIR = {2: 38, 3: 43}
-FLOPS_PER_CANDIDATE = {2: 5, 3: 10}
+# reciprocal square root or reciprocal 1).  Per neighbour pair, in 2D: rsqrt
+# 1, r 1, the clamped factor 3, its cube 2, v_ab . r_ab 6, density difference
+# 1, diffusion 3, continuity sum 2, Monaghan term 8, momentum coefficient 3,
+# its sum 4; in 3D two more operations for every sum over axes (v_ab . r_ab
+# 3, momentum 2) and 7 for c and 1/rho.  Per list entry: the difference d
+# (an integer subtraction and a conversion, counted as one) and |r_ab|^2 2d.
+FLOPS_PER_PAIR = {2: 34, 3: 46}
+FLOPS_PER_CANDIDATE = {2: 6, 3: 9}
 SM_COUNT = 152
 FP32_LANES_PER_SM = 128
 ISSUE_PER_SM_CLK = 4
@@ -267,7 +268,7 @@ def forces_compute(dim: int, n_fluid: int, pairs: int, avg_ms: float,
 
 
 def forces_ceiling(dim: int, form: str) -> dict | None:
-    """The unit that bounds k_forces in its ncu capture (issue slots for the
+    """The unit that bounds k_list_forces in its ncu capture (issue slots for the
     compensated form, the FP64 pipe for the plain one) and how busy it was:
     a recorded capture, beside the live HBM fraction."""
     d = _forces_profile(dim, form)
@@ -613,7 +614,7 @@ def run_gpu(args, ranks) -> dict | None:
     forces_avg_ms = prof32["forces_ms"] / max(prof32["forces_launches"], 1)
     alg = nf * 3 * state_bytes(dim, "fp32c")
     achieved = alg / (forces_avg_ms / 1e3) / 1e9
-    roofline = {"bound": "hbm", "kernel": "k_forces (fused continuity+momentum+RK update)",
+    roofline = {"bound": "hbm", "kernel": "k_list_forces (fused continuity+momentum+RK update)",
                 "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / peaks["hbm_gbs"],
                 "traffic": forces_traffic(dim, "fp32c", nf),
