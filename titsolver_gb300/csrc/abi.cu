@@ -469,8 +469,12 @@ int upload_particles(tg_context* ctx, int32_t n_tanks, const tg_tank* tanks,
     // stays within k cells while particles move 2.5% of R per step, and the
     // outer ring of rows need not be looked at (sort + build 1.23 -> 1.19 ms
     // at 2M fluid particles in 3D, .385 -> .354 at 1.28M in 2D; 3% and 7%
-    // gained less).
-    const double cs = R / C.k * (1.0 + 1.0 / 20.0);
+    // gained less).  The integrators without lists walk cells of R / k
+    // (ms per step on the wider cells and on these: symplectic Euler, 3D 432k
+    // fluid compensated 1.230 / 1.174, 2D 500k .603 / .561, FP64 3D 128k
+    // 7.87 / 7.18; Verlet there 1.854 / 1.772, .897 / .837, 12.05 / 10.93).
+    const bool ssprk = C.P.integrator == TG_SSPRK3 || C.P.integrator == TG_SSPRK2;
+    const double cs = R / C.k * (ssprk ? 1.0 + 1.0 / 20.0 : 1.0 + 1.0 / 65536.0);
     double lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
     if (nt > 0) {
       for (int k = 0; k < dim; ++k) lo[k] = hi[k] = r[base * dim + k];
