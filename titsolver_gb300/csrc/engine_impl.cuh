@@ -584,8 +584,9 @@ class Engine final : public EngineBase {
   // 16 lanes take a 2D list at once).  More lanes repeat the update's FP64
   // operations for fewer particles per warp.  Measured in us per pass, 16 / 4
   // / 1 lanes: 800 fluid particles FP64 with shifting, 1 step 292 / 397 / 722;
-  // 12,800 FP64, 10 steps 4426 / 3965 / 4489; 62,000 compensated with
-  // shifting, 4 steps - / 3311 / 3200.  A launch shape that asks for several
+  // 12,800 FP64, 10 steps 4426 / 3965 / 4489 (later, 4 / 2 / 1 lanes in the
+  // pair sums alone: 3583 / 4136 / 4191); 62,000 compensated with shifting,
+  // 4 steps - / 3311 / 3200.  A launch shape that asks for several
   // lanes gets at least 4.
   static int list_team(const Context& C) {
     const int64_t warps = 4 * static_cast<int64_t>(C.sm_count > 0 ? C.sm_count : 152);

@@ -852,8 +852,8 @@ __device__ __forceinline__ unsigned face_skip_edges(const FaceArgs& fc, uint32_t
 // Lanes per face particle.  3D: a warp (its triangles' edges are shared out
 // over one).  2D: a particle has about nine segments within reach, so a warp
 // takes two particles (pool of 12,800 fluid particles, four steps: 4490 us
-// with 16 lanes, 5577 with 32, 5224 with 8, 5512 with 4: the fewer lanes, the
-// longer each particle's chain of FP64 operations).
+// with 16 lanes, 5577 with 32, 5224 with 8, 5512 with 4, at that time: the
+// fewer lanes, the longer each particle's chain of FP64 operations).
 template<int D>
 constexpr int face_group() {
   return D == 2 ? 16 : 32;

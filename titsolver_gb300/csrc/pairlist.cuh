@@ -1069,9 +1069,10 @@ __device__ __forceinline__ void list_epilogue(const ListArgs<D, F>& A, int64_t i
 }
 
 // Launch bounds (128-thread blocks per SM) and records in flight per lane of
-// the pair loop.  FP64: its pipe is the limit.  Compensated: the gathers take
-// two thirds of L1's wavefronts and the pairs three fifths of the issue slots
-// at the same time.  Measured for the three passes of a step (in a chain of
+// the pair loop.  FP64: its pipe is the limit (87% busy).  Compensated: the
+// gathers take 80% of the L1's throughput and the pairs 56% of the issue slots
+// at the same time (3D 2M fluid: 0.470 ms per launch, 1.448 for the walk over
+// cells).  Measured for the three passes of a step (in a chain of
 // two) at 2M (3D) / 1.28M (2D) fluid particles in ms, blocks x records: 3D
 // 7 x 2 1.59, 6 x 4 1.585, 8 x 2 1.62, 6 x 2 1.62, 9 x 2 1.75, 5 x 4 1.69,
 // 8 x 1 1.68; 2D 9 x 2 .631, 8 x 2 .642, 10 x 2 .665, 7 x 2 .656, 8 x 4 .638,
