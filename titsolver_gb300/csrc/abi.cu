@@ -45,13 +45,17 @@ void Context::release(void* p) {
   allocations.erase(it);
 }
 
+void Context::drop_lists() {
+  list_buf.drop([this](void* p) { release(p); });
+}
+
 void Context::release_all() {
   invalidate_graph();
   if (h_status != nullptr) cudaFreeHost(h_status);
   h_status = nullptr;
-  d_list = d_list_cnt = nullptr;
+  list_buf = ListBuffers{};
   d_vmax = nullptr;
-  lists = false;
+  lists = lists_refused = false;
   list_redos = 0;
   list_cap_scale = 1.0;
   list_margin = 0.005f;
@@ -796,7 +800,7 @@ int tg_step(tg_context* ctx, int32_t n_steps, double* dt_out) {
   const bool steps = n_steps > 0 && C.n > 0;
   if (steps) {
     const bool had = C.lists;
-    TG_CUDA(&C, C.engine->prepare_lists(C));
+    C.engine->prepare_lists(C);
     if (C.lists != had) C.invalidate_graph();
     C.prof.steps += n_steps;
     // With shifting, the post-integration prepare left the walls as the
@@ -834,9 +838,7 @@ int tg_step(tg_context* ctx, int32_t n_steps, double* dt_out) {
     if ((why & tg::kStopMoved) != 0u) C.list_margin *= 2.f;
     if ((why & tg::kStopCapacity) != 0u) {
       C.list_cap_scale *= 1.5;
-      C.release(C.d_list);
-      C.release(C.d_list_cnt);
-      C.d_list = C.d_list_cnt = nullptr;
+      C.drop_lists();
     }
     direct = true;
   }

@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include "faces.cuh"
+#include "listbuf.cuh"
 
 namespace tg {
 
@@ -76,7 +77,7 @@ struct EngineBase {
                                       uint64_t* hashes) = 0;
   // Allocate the step's neighbour lists if it runs on them and has none yet
   // (C.lists says whether it does).
-  virtual cudaError_t prepare_lists(Context& C) = 0;
+  virtual void prepare_lists(Context& C) = 0;
   // Whether the force pass has a variant with `team` lanes per target.
   virtual bool supports_team(int team) const = 0;
 };
@@ -192,15 +193,17 @@ struct Context {
   int64_t graph_kernels[2][2] = {};
 
   // Neighbour lists of the step (pairlist.cuh): whether steps run on them,
-  // their capacity per particle, the acceleration margin and how often a
-  // step had to be repeated (lists_max_redo: no lists until the next upload).
+  // whether there is no room for them (decided once, so that the route does
+  // not change between calls with what others leave of the memory), their
+  // capacity per particle, the acceleration margin and how often a step had
+  // to be repeated (past kListMaxRedos: no lists until the next upload).
   bool lists = false;
+  bool lists_refused = false;
   int list_cap = 0;
   double list_cap_scale = 1.0;
   float list_margin = 0.005f;
   int list_redos = 0;
-  uint32_t* d_list = nullptr;
-  uint32_t* d_list_cnt = nullptr;
+  ListBuffers list_buf;
 
   bool walls_fresh = false;
   bool keys_valid = false;  // home keys match the home positions
@@ -217,6 +220,7 @@ struct Context {
 
   cudaError_t alloc(void** p, size_t bytes);
   void release(void* p);  // one buffer of alloc
+  void drop_lists();
   void release_all();
   void invalidate_graph();
 

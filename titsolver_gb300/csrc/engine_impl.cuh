@@ -84,9 +84,6 @@ class Engine final : public EngineBase {
       }
       A(U.rho, n);
     }
-    posrec_b_ = nullptr;
-    datrec_b_ = nullptr;
-    travel_ = nullptr;
     // Two spare records: the staged force pass copies row segments rounded
     // out to 16-byte boundaries, which may reach one record past the end.
     A(posrec_, n + 2);
@@ -125,58 +122,12 @@ class Engine final : public EngineBase {
     return cudaGetLastError();
   }
 
-  cudaError_t prepare_lists(Context& C) override {
+  void prepare_lists(Context& C) override {
     C.lists = false;
     const bool rk = C.P.integrator == TG_SSPRK2 || C.P.integrator == TG_SSPRK3;
-    if (!rk || C.n == 0 || C.n_fluid == 0 || C.list_redos >= kListMaxRedos) return cudaSuccess;
-    if (C.d_list == nullptr) {
-      // Entries per particle: those of a ball of the list's radius at the
-      // reference density, with room for disorder and compression; the
-      // largest over the tanks.
-      double most = 0.0;
-      for (size_t t = 0; t < C.tanks.size(); ++t) {
-        const TankDev& T = C.tankdev[t];
-        const double R = 1.1 * T.R_f;
-        const double ball = D == 2 ? 3.14159265358979 * R * R : 4.18879020478639 * R * R * R;
-        most = std::max(most, ball * T.rho0 / T.m);
-        // Tank-local FP32 coordinates must resolve the radius.
-        if (T.list_slack_f > 0.02f * T.R_f) return cudaSuccess;
-      }
-      const double cap = std::ceil((1.3 * most + 12.0) * C.list_cap_scale / 4.0) * 4.0;
-      const int64_t tiles = (C.n + 31) / 32;
-      const double bytes = 32.0 * static_cast<double>(tiles) *
-                           (4.0 * cap + sizeof(uint32_t) + sizeof(DatRec) + sizeof(PosRec));
-      size_t avail = 0, total = 0;
-      if (cudaMemGetInfo(&avail, &total) != cudaSuccess) {
-        cudaGetLastError();
-        return cudaSuccess;
-      }
-      // Lists are an option: they leave most of the memory to others.
-      if (!(cap <= kListMaxCap) || bytes > 0.35 * static_cast<double>(avail)) return cudaSuccess;
-      C.list_cap = static_cast<int>(cap);
-      cudaError_t e = C.alloc(reinterpret_cast<void**>(&C.d_list),
-                              sizeof(uint32_t) * 32 * static_cast<size_t>(tiles) * C.list_cap);
-      if (e == cudaSuccess) {
-        e = C.alloc(reinterpret_cast<void**>(&C.d_list_cnt), sizeof(uint32_t) * C.n);
-      }
-      if (e == cudaSuccess && datrec_b_ == nullptr) {
-        // The list build reads a few 16-byte records past the last.
-        e = C.alloc(reinterpret_cast<void**>(&datrec_b_), sizeof(DatRec) * (C.n + kListScan));
-        if (e == cudaSuccess && F == TG_FP64) {
-          e = C.alloc(reinterpret_cast<void**>(&posrec_b_), sizeof(PosRec) * C.n);
-        }
-        if (e == cudaSuccess) {
-          e = C.alloc(reinterpret_cast<void**>(&travel_), sizeof(float) * C.n);
-        }
-      }
-      if (e != cudaSuccess) {
-        cudaGetLastError();
-        release_lists(C);
-        return cudaSuccess;
-      }
-    }
-    C.lists = true;
-    return cudaSuccess;
+    if (!rk || C.n == 0 || C.n_fluid == 0 || C.list_redos >= kListMaxRedos) return;
+    if (!C.list_buf.held() && !C.lists_refused) C.lists_refused = !take_lists(C);
+    C.lists = C.list_buf.held();
   }
 
   int chain(const Context& C) const override {
@@ -396,11 +347,45 @@ class Engine final : public EngineBase {
     return cudaGetLastError();
   }
 
-  void release_lists(Context& C) {
-    C.release(C.d_list);
-    C.release(C.d_list_cnt);
-    C.d_list = nullptr;
-    C.d_list_cnt = nullptr;
+  // Takes the buffers of the list steps; false where they do not fit.
+  bool take_lists(Context& C) {
+    // Entries per particle: those of a ball of the list's radius at the
+    // reference density, with room for disorder and compression; the
+    // largest over the tanks.
+    double most = 0.0;
+    for (size_t t = 0; t < C.tanks.size(); ++t) {
+      const TankDev& T = C.tankdev[t];
+      const double R = 1.1 * T.R_f;
+      const double ball = D == 2 ? 3.14159265358979 * R * R : 4.18879020478639 * R * R * R;
+      most = std::max(most, ball * T.rho0 / T.m);
+      // Tank-local FP32 coordinates must resolve the radius.
+      if (T.list_slack_f > 0.02f * T.R_f) return false;
+    }
+    const double cap = std::ceil((1.3 * most + 12.0) * C.list_cap_scale / 4.0) * 4.0;
+    if (!(cap <= kListMaxCap)) return false;
+    C.list_cap = static_cast<int>(cap);
+    const size_t n = static_cast<size_t>(C.n), slots = 32 * ((n + 31) / 32);
+    size_t bytes[kListBufs] = {};
+    bytes[kListEntries] = sizeof(uint32_t) * slots * static_cast<size_t>(C.list_cap);
+    bytes[kListCounts] = sizeof(uint32_t) * n;
+    // The list build reads a few 16-byte records past the last.
+    bytes[kListDat] = sizeof(DatRec) * (n + kListScan);
+    bytes[kListPos] = F == TG_FP64 ? sizeof(PosRec) * n : 0;
+    bytes[kListTravel] = sizeof(float) * n;
+    size_t all = 0, avail = 0, total = 0;
+    for (const size_t b : bytes) all += b;
+    // Lists are an option: they leave most of the memory to others.
+    const bool fits = cudaMemGetInfo(&avail, &total) == cudaSuccess &&
+                      static_cast<double>(all) <= 0.35 * static_cast<double>(avail);
+    const bool taken = fits && C.list_buf.take(
+        bytes,
+        [&C](size_t size) {
+          void* p = nullptr;
+          return C.alloc(&p, size) == cudaSuccess ? p : nullptr;
+        },
+        [&C](void* p) { C.release(p); });
+    if (!taken) cudaGetLastError();
+    return taken;
   }
 
   // Steps on neighbour lists (pairlist.cuh): one sort, lists for all their
@@ -415,9 +400,12 @@ class Engine final : public EngineBase {
     A.dat_in = datrec_;
     for (int k = 0; k < D; ++k) A.pin[k] = Y_.pos[k];
     // Read by the list build only, before the first stage writes these.
-    A.lrec = reinterpret_cast<float4*>(datrec_b_);
-    A.list = C.d_list;
-    A.cnt = C.d_list_cnt;
+    auto* datrec_b = static_cast<DatRec*>(C.list_buf.p[kListDat]);
+    auto* posrec_b = static_cast<PosRec*>(C.list_buf.p[kListPos]);
+    auto* travel = static_cast<float*>(C.list_buf.p[kListTravel]);
+    A.lrec = reinterpret_cast<float4*>(datrec_b);
+    A.list = static_cast<uint32_t*>(C.list_buf.p[kListEntries]);
+    A.cnt = static_cast<uint32_t*>(C.list_buf.p[kListCounts]);
     // The face passes need the current cells; the sort's payload buffer that
     // does not hold the permutation is free after the gather, and so is the
     // permutation.
@@ -465,7 +453,7 @@ class Engine final : public EngineBase {
         for (int k = 0; k < D; ++k) A.S.Y.pos[k] = pos[start][k];
         A.S.Udst = U_[step & 1];
         A.S.dt = C.d_dt + static_cast<size_t>(step) * C.ntanks;
-        A.travel = step > 0 ? travel_ : nullptr;
+        A.travel = step > 0 ? travel : nullptr;
       }
       A.first = q == 0;
       A.carry = end && step + 1 < steps;
@@ -474,15 +462,15 @@ class Engine final : public EngineBase {
       if (A.carry) {
         A.next = U_[(step + 1) & 1];
         A.dt_next = A.S.dt + C.ntanks;
-        A.travel_out = travel_;
+        A.travel_out = travel;
       }
       A.S.lincomb = s > 0;
       A.S.w_new = (stages == 2 ? w2 : w3)[s];
       A.w0 = 1.0 - A.S.w_new;
       A.wr = static_cast<R>(A.S.w_new);
       A.w0r = static_cast<R>(A.w0);
-      A.pos_out = reinterpret_cast<typename ListArgs<D, F>::PosRec*>(in_b ? posrec_ : posrec_b_);
-      A.dat_out = in_b ? datrec_ : datrec_b_;
+      A.pos_out = reinterpret_cast<typename ListArgs<D, F>::PosRec*>(in_b ? posrec_ : posrec_b);
+      A.dat_out = in_b ? datrec_ : datrec_b;
       in_b = !in_b;
       const int out = (start + 1 + (s & 1)) % 3;
       for (int k = 0; k < D; ++k) A.pout[k] = pos[out][k];
@@ -869,9 +857,6 @@ class Engine final : public EngineBase {
   PostArgs<D, F> post_{};
   PosRec* posrec_ = nullptr;
   DatRec* datrec_ = nullptr;
-  PosRec* posrec_b_ = nullptr;  // the list step's second records
-  DatRec* datrec_b_ = nullptr;
-  float* travel_ = nullptr;     // paths within a chain of steps
 };
 
 template <int D, int F, int K>
