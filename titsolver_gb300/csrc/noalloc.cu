@@ -214,25 +214,25 @@ __global__ void __launch_bounds__(256)
   keys[i] = key_of(flat_cell<D>(*T, c), false);
 }
 
+// perm_z: the permutation, and in 3D then the local z coordinates in its place
+// (entry j is read and written by the thread of j only).
 template<int D>
 __global__ void __launch_bounds__(256)
-    k_na_records(const double* __restrict__ r, const uint32_t* __restrict__ perm, int64_t n,
+    k_na_records(const double* __restrict__ r, uint32_t* __restrict__ perm_z, int64_t n,
                  const TankDev* __restrict__ T, void* __restrict__ recs,
-                 uint32_t* __restrict__ ids, float* __restrict__ lx, float* __restrict__ ly,
-                 float* __restrict__ lz) {
+                 uint32_t* __restrict__ ids, float* __restrict__ lx, float* __restrict__ ly) {
   const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (j >= n) return;
-  const uint32_t s = perm[j];
+  const uint32_t s = perm_z[j];
   const double* p = r + static_cast<int64_t>(s) * D;
   ids[j] = s;
-  // lz may be the buffer of perm, whose entry j was read above.
   lx[j] = __double2float_rn(p[0] - T->lo[0]);
   ly[j] = __double2float_rn(p[1] - T->lo[1]);
   if constexpr (D == 2) {
     static_cast<Pos64_2*>(recs)[j] = Pos64_2{p[0], p[1]};
   } else {
     static_cast<Pos64_3*>(recs)[j] = Pos64_3{p[0], p[1], p[2], 0.0};
-    lz[j] = __double2float_rn(p[2] - T->lo[2]);
+    perm_z[j] = __float_as_uint(__double2float_rn(p[2] - T->lo[2]));
   }
 }
 
@@ -265,15 +265,15 @@ cudaError_t run(unsigned char* base, int64_t n, const double* r, double h,
                              base + kOffHist, &in_b, s, &launches);
   if (e != cudaSuccess) return e;
   const uint32_t* sorted = in_b ? keys_b : keys_a;
-  const uint32_t* perm = in_b ? vals_b : vals_a;
+  uint32_t* perm = in_b ? vals_b : vals_a;
   e = build_cell_table(sorted, n, 2 * kMaxCells, cells, base + kOffBounds, s, &launches);
   if (e != cudaSuccess) return e;
   // The sort's other buffers, and the permutation's own, take the local
   // coordinates.
   auto* lx = reinterpret_cast<float*>(in_b ? keys_a : keys_b);
   auto* ly = reinterpret_cast<float*>(in_b ? vals_a : vals_b);
-  auto* lz = reinterpret_cast<float*>(in_b ? vals_b : vals_a);
-  k_na_records<D><<<g, 256, 0, s>>>(r, perm, n, T, recs, ids, lx, ly, lz);
+  k_na_records<D><<<g, 256, 0, s>>>(r, perm, n, T, recs, ids, lx, ly);
+  auto* lz = reinterpret_cast<float*>(perm);
   // One tank whose first cell (and first id) is 0: id_base doubles as the
   // tank cell-offset table.
   const CloudArgs<D> a{recs, {lx, ly, lz}, nullptr, ids, sorted, cells, T, id_base, 1, n, 0,
