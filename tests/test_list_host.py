@@ -10,7 +10,7 @@ import pytest
 ROOT = pathlib.Path(__file__).resolve().parent.parent
 
 
-@pytest.mark.parametrize("name", ("list_buffers",))
+@pytest.mark.parametrize("name", ("list_buffers", "list_policy"))
 def test_list_host(tmp_path, name):
     exe = tmp_path / name
     subprocess.run(["g++", "-std=c++20", "-O1", "-Wall", "-Wextra", "-Werror",

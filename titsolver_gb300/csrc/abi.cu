@@ -56,9 +56,7 @@ void Context::release_all() {
   list_buf = ListBuffers{};
   d_vmax = nullptr;
   lists = lists_refused = false;
-  list_redos = 0;
-  list_cap_scale = 1.0;
-  list_margin = 0.005f;
+  list_policy = ListPolicy{};
   for (void* p : allocations) cudaFree(p);
   allocations.clear();
   d_tanks = nullptr;
@@ -83,9 +81,9 @@ void Context::release_all() {
   keys_valid = false;
 }
 
-void Context::invalidate_graph() {
-  for (auto& per_length : graph_exec) {
-    for (cudaGraphExec_t& g : per_length) {
+void Context::invalidate_graph(int first, int last) {
+  for (int l = first; l <= last; ++l) {
+    for (cudaGraphExec_t& g : graph_exec[l]) {
       if (g != nullptr) cudaGraphExecDestroy(g);
       g = nullptr;
     }
@@ -745,7 +743,7 @@ int tg_prepare(tg_context* ctx) {
 namespace {
 
 // Enqueue n steps: graph replays (captured on first use), or direct launches
-// while profiling, without graphs, or where a stopped step is repeated.
+// while profiling, without graphs, or where a few stopped steps are repeated.
 int enqueue_steps(Context& C, int32_t n, bool direct) {
   TG_CUDA(&C, C.engine->ensure_keys(C));
   const int chain = C.engine->chain(C);
@@ -760,7 +758,7 @@ int enqueue_steps(Context& C, int32_t n, bool direct) {
     }
     // The re-sort is taken only in the home order of an earlier sort, a
     // host-side choice baked into the graph: one graph for each.
-    const int l = steps > 1 ? 1 : 0, o = C.order_valid ? 1 : 0;
+    const int l = !C.lists ? 2 : steps > 1 ? 1 : 0, o = C.order_valid ? 1 : 0;
     cudaGraphExec_t& exec = C.graph_exec[l][o];
     if (exec == nullptr) {
       cudaGraph_t graph = nullptr;
@@ -787,6 +785,28 @@ int enqueue_steps(Context& C, int32_t n, bool direct) {
   return TG_OK;
 }
 
+// Wait for the enqueued steps and read the status words and the time steps:
+// how many steps were finished since the last call, and why one was stopped
+// (0: none was).  It and those behind it left the state alone.
+int settle(Context& C, uint32_t* done, uint32_t* why) {
+  auto* status = static_cast<uint32_t*>(C.h_status);
+  TG_CUDA(&C, cudaMemcpyAsync(status, C.d_err, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                              C.stream));
+  TG_CUDA(&C, cudaMemcpyAsync(status + 4, C.d_dt_last, sizeof(double) * C.ntanks,
+                              cudaMemcpyDeviceToHost, C.stream));
+  TG_CUDA(&C, cudaStreamSynchronize(C.stream));
+  C.drain_profile();
+  *done = status[2] - C.steps_done;
+  C.steps_done = status[2];
+  *why = status[1];
+  if (*why != 0u) {
+    TG_CUDA(&C, cudaMemsetAsync(C.d_err + 1, 0, sizeof(uint32_t), C.stream));
+    C.keys_valid = false;
+    C.order_valid = false;
+  }
+  return TG_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -795,53 +815,46 @@ int tg_step(tg_context* ctx, int32_t n_steps, double* dt_out) {
   if (ctx == nullptr || n_steps < 0) return TG_ERR_INVALID_ARGUMENT;
   Context& C = ctx->c;
   if (!C.uploaded) return fail(&C, TG_ERR_NOT_READY, "no particles uploaded");
-  auto* status = static_cast<uint32_t*>(C.h_status);
-  auto* last_dt = reinterpret_cast<double*>(status + 4);
-  const bool steps = n_steps > 0 && C.n > 0;
-  if (steps) {
-    const bool had = C.lists;
-    C.engine->prepare_lists(C);
-    if (C.lists != had) C.invalidate_graph();
+  const auto* status = static_cast<const uint32_t*>(C.h_status);
+  const auto* last_dt = reinterpret_cast<const double*>(status + 4);
+  int32_t left = C.n > 0 ? n_steps : 0;
+  if (left > 0) {
     C.prof.steps += n_steps;
     // With shifting, the post-integration prepare left the walls as the
     // reference leaves them (extrapolated before the shift); otherwise the
     // reference's closing prepare runs on the next density download.
     C.walls_fresh = C.P.post_integrate == TG_POST_SHIFTING;
   }
-  bool direct = !C.use_graph || C.profile;
-  int32_t left = steps ? n_steps : 0;
-  for (;;) {
-    if (left > 0) {
-      const int st = enqueue_steps(C, left, direct);
-      if (st != TG_OK) return st;
-    }
-    TG_CUDA(&C, cudaMemcpyAsync(status, C.d_err, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                C.stream));
-    TG_CUDA(&C, cudaMemcpyAsync(last_dt, C.d_dt_last, sizeof(double) * C.ntanks,
-                                cudaMemcpyDeviceToHost, C.stream));
-    TG_CUDA(&C, cudaStreamSynchronize(C.stream));
-    C.drain_profile();
-    const uint32_t done = status[2] - C.steps_done;
-    C.steps_done = status[2];
-    if (status[1] == 0u) break;
-    // A step could not be finished on its lists (pairlist.cuh): it and those
-    // behind it left the state alone.  The rest of this call sorts in every
-    // stage; later calls get longer lists or a wider margin.
-    const uint32_t why = status[1];
-    left -= static_cast<int32_t>(done);
-    TG_CUDA(&C, cudaMemsetAsync(C.d_err + 1, 0, sizeof(uint32_t), C.stream));
-    C.keys_valid = false;
-    C.order_valid = false;
+  tg::ListPolicy& policy = C.list_policy;
+  do {
+    const bool walk = policy.walk > 0;
     C.lists = false;
-    C.invalidate_graph();
-    C.list_redos += 1;
-    if ((why & tg::kStopMoved) != 0u) C.list_margin *= 2.f;
-    if ((why & tg::kStopCapacity) != 0u) {
-      C.list_cap_scale *= 1.5;
-      C.drop_lists();
+    if (left > 0 && !walk) C.engine->prepare_lists(C);
+    const int32_t batch = walk ? std::min(left, policy.walk)
+                          : C.lists ? std::min(left, policy.batch)
+                                    : left;
+    // A graph of the walk pays from a few steps on.
+    const bool direct = !C.use_graph || C.profile ||
+                        (walk && batch < 4 && C.graph_exec[2][1] == nullptr);
+    const int st = batch > 0 ? enqueue_steps(C, batch, direct) : TG_OK;
+    uint32_t done = 0, why = 0;
+    const int settled = settle(C, &done, &why);
+    if (st != TG_OK) return st;
+    if (settled != TG_OK) return settled;
+    if (why != 0u) {
+      left -= static_cast<int32_t>(done);
+      policy.stopped(why, std::min(left, C.engine->chain(C)));
+      C.invalidate_graph(0, 1);
+      if ((why & tg::kStopCapacity) != 0u) C.drop_lists();
+      continue;
     }
-    direct = true;
-  }
+    left -= batch;
+    if (walk) {
+      policy.walked(batch);
+    } else if (C.lists && policy.finished(batch)) {
+      C.invalidate_graph(0, 1);
+    }
+  } while (left > 0);
   if (dt_out != nullptr) std::memcpy(dt_out, last_dt, sizeof(double) * C.ntanks);
   const uint32_t err = status[0];
   if (err & (TG_DEV_NONFINITE_STATE | TG_DEV_BAD_DT)) {
@@ -1639,6 +1652,9 @@ int tg_autotune(tg_context* ctx, int32_t trial_steps, tg_tuning* out) {
   tg_get_tuning(ctx, &best);
   best.ms_per_step = std::numeric_limits<double>::infinity();
   int timed = 0;
+  // Steps that trials have to repeat neither bias the next ones nor stay with
+  // the context.
+  const tg::ListPolicy policy = C.list_policy;
   // Time `trial_steps` graph-replayed steps of one shape (one untimed step
   // first captures the graph); the state goes back afterwards.
   auto trial = [&](tg_tuning t, double* ms) -> int {
@@ -1648,6 +1664,7 @@ int tg_autotune(tg_context* ctx, int32_t trial_steps, tg_tuning* out) {
     if (s != TG_OK) return s;
     C.force_block = t.block_size;
     C.force_team = t.lanes_per_particle;
+    C.list_policy = tg::ListPolicy{};
     C.invalidate_graph();
     s = tg_step(ctx, 1, nullptr);
     if (s == TG_OK) s = tg_timer_start(ctx);
@@ -1695,6 +1712,7 @@ int tg_autotune(tg_context* ctx, int32_t trial_steps, tg_tuning* out) {
   // Leave the context at the best shape with the state of the call.
   const int st2 = restore_snapshot(
       ctx, S, std::isfinite(best.ms_per_step) ? best.cells_per_radius : C.k);
+  C.list_policy = policy;
   if (st != TG_OK) return st;
   if (st2 != TG_OK) return st2;
   if (!std::isfinite(best.ms_per_step)) {

@@ -11,6 +11,7 @@
 
 #include "faces.cuh"
 #include "listbuf.cuh"
+#include "listpolicy.cuh"
 
 namespace tg {
 
@@ -22,10 +23,6 @@ struct Context;
 // 2.44 / 3.02 / 3.03, 24 3D tanks 1.68 / 1.39 / 1.84 / 1.98, 2D 1.28M 0.969 /
 // 0.854 / 0.849 / 0.815.
 constexpr int kListChain = 2;
-
-// Why a step could not be finished on its neighbour lists (status word [1]).
-constexpr uint32_t kStopMoved = 1u;     // a particle moved beyond the bound
-constexpr uint32_t kStopCapacity = 2u;  // a list outgrew its capacity
 
 // Force passes per step of an integrator.
 inline int force_passes(int integrator) {
@@ -186,23 +183,22 @@ struct Context {
   const uint32_t* sorted_keys = nullptr;
   const uint32_t* perm = nullptr;
 
-  // CUDA graphs of one step [0] and of a chain [1], each from a home state
-  // out of order (full sort) [0] and in the order of its last sort [1].
+  // CUDA graphs of one step on lists [0], of a chain [1] and of one step that
+  // walks cells [2], each from a home state out of order (full sort) [0] and
+  // in the order of its last sort [1].
   bool use_graph = true;
-  cudaGraphExec_t graph_exec[2][2] = {};
-  int64_t graph_kernels[2][2] = {};
+  cudaGraphExec_t graph_exec[3][2] = {};
+  int64_t graph_kernels[3][2] = {};
 
   // Neighbour lists of the step (pairlist.cuh): whether steps run on them,
   // whether there is no room for them (decided once, so that the route does
   // not change between calls with what others leave of the memory), their
-  // capacity per particle, the acceleration margin and how often a step had
-  // to be repeated (past kListMaxRedos: no lists until the next upload).
+  // capacity per particle, and what follows from steps that had to be
+  // repeated.
   bool lists = false;
   bool lists_refused = false;
   int list_cap = 0;
-  double list_cap_scale = 1.0;
-  float list_margin = 0.005f;
-  int list_redos = 0;
+  ListPolicy list_policy;
   ListBuffers list_buf;
 
   bool walls_fresh = false;
@@ -222,7 +218,7 @@ struct Context {
   void release(void* p);  // one buffer of alloc
   void drop_lists();
   void release_all();
-  void invalidate_graph();
+  void invalidate_graph(int first = 0, int last = 2);
 
   // Profiling helpers (no-ops unless profile is on and not capturing).
   int group_begin(int group);

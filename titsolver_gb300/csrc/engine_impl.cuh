@@ -31,10 +31,8 @@ inline int physics_preset(const tg_params& P) {
   return kPhysGeneric;
 }
 
-// Longest list of a particle, and how many steps may have to be repeated
-// before a context goes without lists until the next upload.
+// Longest list of a particle.
 constexpr double kListMaxCap = 1024.0;
-constexpr int kListMaxRedos = 4;
 
 // Kernels with multi-lane force variants: the two the shipped parameter
 // sets use (Wendland C2 and C4); the others run one lane per target.
@@ -125,15 +123,14 @@ class Engine final : public EngineBase {
   void prepare_lists(Context& C) override {
     C.lists = false;
     const bool rk = C.P.integrator == TG_SSPRK2 || C.P.integrator == TG_SSPRK3;
-    if (!rk || C.n == 0 || C.n_fluid == 0 || C.list_redos >= kListMaxRedos) return;
+    if (!rk || C.n == 0 || C.n_fluid == 0) return;
     if (!C.list_buf.held() && !C.lists_refused) C.lists_refused = !take_lists(C);
     C.lists = C.list_buf.held();
   }
 
   int chain(const Context& C) const override {
-    // Not where the FP64 pipe would pay for every further entry, nor after a
-    // step of this context had to be repeated.
-    return (F == TG_FP32C || list_team(C) > 1) && C.lists && C.list_redos == 0 &&
+    // Not where the FP64 pipe would pay for every further entry.
+    return (F == TG_FP32C || list_team(C) > 1) && C.lists && C.list_policy.chains &&
                    C.P.post_integrate != TG_POST_SHIFTING && !C.faces.on
                ? kListChain
                : 1;
@@ -361,7 +358,7 @@ class Engine final : public EngineBase {
       // Tank-local FP32 coordinates must resolve the radius.
       if (T.list_slack_f > 0.02f * T.R_f) return false;
     }
-    const double cap = std::ceil((1.3 * most + 12.0) * C.list_cap_scale / 4.0) * 4.0;
+    const double cap = std::ceil((1.3 * most + 12.0) * C.list_policy.room / 4.0) * 4.0;
     if (!(cap <= kListMaxCap)) return false;
     C.list_cap = static_cast<int>(cap);
     const size_t n = static_cast<size_t>(C.n), slots = 32 * ((n + 31) / 32);
@@ -414,7 +411,7 @@ class Engine final : public EngineBase {
     A.stop = C.d_err + 1;
     A.n_walls = C.n_wall;
     A.cap = C.list_cap;
-    A.margin = C.list_margin;
+    A.margin = C.list_policy.margin;
     A.chain = steps;
     A.dt_build = C.d_dt;
     int tok = C.group_begin(kGroupReorder);
