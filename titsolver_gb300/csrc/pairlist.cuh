@@ -708,7 +708,7 @@ struct ListPairF32 {
         const float xr = fmaf(b.drho, inv_rho0, 1.f);
         cb = cs0 * (xr * xr * xr);
       }
-      ib = rcp_approx(rho0 + b.drho);
+      ib = rcp_newton(rho0 + b.drho);
     }
     const float rinv = rsqrt_seed(s2);
     const float r = s2 * rinv;
@@ -902,8 +902,8 @@ __global__ void __launch_bounds__(128) k_list_walls(ListArgs<D, F> A) {
           const float s2 = own.rab(b, d);
           if (s2 > T.list_hi_f) continue;
           if (s2 >= T.list_lo_f && !within_fp64<D>(A.pin, ew, js[q], T.radius2)) continue;
-          const float W = T.w_f * KernelPoly<K>::value(sqrt_approx(s2) * hq);
-          const float ib = D == 2 ? b.invrho : rcp_approx(T.rho0_f + b.drho);
+          const float W = T.w_f * KernelPoly<K>::value(sqrt_newton(s2) * hq);
+          const float ib = D == 2 ? b.invrho : rcp_newton(T.rho0_f + b.drho);
           const float Vb = T.m_f * ib;
           float Hb = potential_f32(S.phys, T, b.drho);
           if (S.fc.on) {
