@@ -93,5 +93,11 @@ int main() {
            const double u = 1.0 + t;
            return std::pow(static_cast<LD>(u), 1.0L / 6.0L);
          });
+  // Zero, and squares that are no normal numbers: no larger than the root.
+  std::vector<double> tiny = {0.0, 4.9e-324, 1e-320, 1e-310, 2.2250738585072009e-308};
+  report("sqrt_f64_tiny", tiny, [] __device__(double x) {
+    const double r = tg::sqrt_f64(x);
+    return r >= 0.0 && r <= 1.0001 * sqrt(x) ? 1.0 : 0.0;
+  }, [](double) { return 1.0L; });
   return 0;
 }

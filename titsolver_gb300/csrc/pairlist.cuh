@@ -752,6 +752,7 @@ struct ListPairF64 {
   double mhinv2, hinv, ah, eps2, dk, mu2;
   double R2;
   int visc, diff, r2hi;
+  unsigned within;  // high words of normal numbers clearly below R^2
   double drho, dv[3];
 
   __device__ __forceinline__ void init(const ListArgs<D, F>& A, const TankDev& T, int64_t i) {
@@ -765,13 +766,16 @@ struct ListPairF64 {
     mu2 = 2.0 * A.S.phys.mu * a.invrho;
     R2 = T.radius2;
     r2hi = __double2hiint(R2);
+    within = static_cast<unsigned>(max(r2hi - 1 - 0x00100000, 0));
     visc = A.S.phys.viscosity;
     diff = A.S.phys.diffusion;
     drho = dv[0] = dv[1] = dv[2] = 0.0;
   }
   // r_ab, |r_ab|^2 and the reference's predicate: decided by the high words
   // except where they are within one of R^2's, there on the reference's own
-  // rounding (dist2_exact).
+  // rounding (dist2_exact).  Particles whose squared distance is a subnormal
+  // number, which the seed would flush, add nothing: the reference's unit
+  // vector is 0 there.
   __device__ __forceinline__ bool near(const double* y, double* d, double& s2) const {
     s2 = 0.0;
 #pragma unroll
@@ -780,7 +784,8 @@ struct ListPairF64 {
       s2 = k == 0 ? d[0] * d[0] : fma(d[k], d[k], s2);
     }
     const int hi = __double2hiint(s2);
-    if (hi < r2hi - 1) return true;
+    if (static_cast<unsigned>(hi - 0x00100000) < within) return true;
+    if (hi < 0x00100000) return s2 == 0.0;
     if (hi > r2hi + 1) return false;
     double t[3];
     return dist2_exact<D>(x, y, t) <= R2;
