@@ -571,12 +571,12 @@ class Engine final : public EngineBase {
   // / 1 lanes: 800 fluid particles FP64 with shifting, 1 step 292 / 397 / 722;
   // 12,800 FP64, 10 steps 4426 / 3965 / 4489 (later, 4 / 2 / 1 lanes in the
   // pair sums alone: 3583 / 4136 / 4191); 62,000 compensated with shifting,
-  // 4 steps - / 3311 / 3200.  A launch shape that asks for several
-  // lanes gets at least 4.
+  // 4 steps - / 3311 / 3200.  The launch shape of a context is that of the
+  // cell walk and does not enter here: neither the lanes nor, through them,
+  // the plain form's chains are its choice.
   static int list_team(const Context& C) {
     const int64_t warps = 4 * static_cast<int64_t>(C.sm_count > 0 ? C.sm_count : 152);
-    if (C.n_fluid < 8 * warps) return 16;
-    return C.n_fluid < 32 * warps || C.force_team > 1 ? 4 : 1;
+    return C.n_fluid < 8 * warps ? 16 : C.n_fluid < 32 * warps ? 4 : 1;
   }
   template<int Team>
   void launch_build(Context& C, const ListArgs<D, F>& A) {
@@ -602,7 +602,7 @@ class Engine final : public EngineBase {
   }
   template<int Phys>
   void launch_list_forces(Context& C, const ListArgs<D, F>& A, int team) {
-    const int block = std::min(C.force_block, 128);
+    constexpr int block = 128;
     // The band lists of the compensated B-spline sums.
     const size_t smem = F == TG_FP32C && !KernelPoly<K>::deriv_over_q
                             ? sizeof(uint32_t) * kBandCap * static_cast<size_t>(block)
