@@ -382,7 +382,9 @@ int tg_set_tuning(tg_context* ctx, const tg_tuning* tuning);
  * the uploaded particles, by coordinate search over cells_per_radius, then
  * lanes_per_particle, then block_size, and leaves the context at the
  * fastest shape with the particle state and clocks of the call (the trial
- * steps are undone).  out (may be NULL) receives the choice. */
+ * steps are undone).  Where steps run on neighbour lists, lanes and blocks
+ * are timed on the cell walk that repeated steps take, and ms_per_step is
+ * that of the steps on lists.  out (may be NULL) receives the choice. */
 int tg_autotune(tg_context* ctx, int32_t trial_steps, tg_tuning* out);
 
 /* Human-readable text of a status code, and of the context's last error. */

@@ -742,8 +742,41 @@ int tg_prepare(tg_context* ctx) {
 
 namespace {
 
-// Enqueue n steps: graph replays (captured on first use), or direct launches
-// while profiling, without graphs, or where a few stopped steps are repeated.
+// The graph of one step, or of a chain, on the route and in the home order of
+// now: captured on first use.  The re-sort is taken only in the home order of
+// an earlier sort, a host-side choice baked into the graph: one for each.
+int step_graph(Context& C, int steps, cudaGraphExec_t* exec, int64_t* kernels) {
+  const int l = !C.lists ? 2 : steps > 1 ? 1 : 0, o = C.order_valid ? 1 : 0;
+  cudaGraphExec_t& kept = C.graph_exec[l][o];
+  if (kept == nullptr) {
+    // Capturing runs nothing: the sort's results and the home state are as
+    // they were.
+    const bool keys = C.keys_valid, order = C.order_valid;
+    cudaGraph_t graph = nullptr;
+    const int64_t before = C.launches;
+    TG_CUDA(&C, cudaStreamBeginCapture(C.stream, cudaStreamCaptureModeThreadLocal));
+    const cudaError_t e = C.engine->enqueue_step(C, steps);
+    const cudaError_t e2 = cudaStreamEndCapture(C.stream, &graph);
+    C.graph_kernels[l][o] = C.launches - before;
+    C.launches = before;
+    C.keys_valid = keys;
+    C.order_valid = order;
+    if (e != cudaSuccess) return cuda_fail(&C, e, "enqueue_step");
+    if (e2 != cudaSuccess) return cuda_fail(&C, e2, "cudaStreamEndCapture");
+    const cudaError_t e3 = cudaGraphInstantiate(&kept, graph, 0);
+    cudaGraphDestroy(graph);
+    if (e3 != cudaSuccess) {
+      kept = nullptr;
+      return cuda_fail(&C, e3, "cudaGraphInstantiate");
+    }
+  }
+  *exec = kept;
+  *kernels = C.graph_kernels[l][o];
+  return TG_OK;
+}
+
+// Enqueue n steps: graph replays, or direct launches while profiling, without
+// graphs, or where a few stopped steps are repeated.
 int enqueue_steps(Context& C, int32_t n, bool direct) {
   TG_CUDA(&C, C.engine->ensure_keys(C));
   const int chain = C.engine->chain(C);
@@ -756,29 +789,12 @@ int enqueue_steps(Context& C, int32_t n, bool direct) {
       C.prof.forces_launches += steps * tg::force_passes(C.P.integrator);
       continue;
     }
-    // The re-sort is taken only in the home order of an earlier sort, a
-    // host-side choice baked into the graph: one graph for each.
-    const int l = !C.lists ? 2 : steps > 1 ? 1 : 0, o = C.order_valid ? 1 : 0;
-    cudaGraphExec_t& exec = C.graph_exec[l][o];
-    if (exec == nullptr) {
-      cudaGraph_t graph = nullptr;
-      const int64_t before = C.launches;
-      TG_CUDA(&C, cudaStreamBeginCapture(C.stream, cudaStreamCaptureModeThreadLocal));
-      const cudaError_t e = C.engine->enqueue_step(C, steps);
-      const cudaError_t e2 = cudaStreamEndCapture(C.stream, &graph);
-      if (e != cudaSuccess) return cuda_fail(&C, e, "enqueue_step");
-      if (e2 != cudaSuccess) return cuda_fail(&C, e2, "cudaStreamEndCapture");
-      C.graph_kernels[l][o] = C.launches - before;
-      C.launches = before;
-      const cudaError_t e3 = cudaGraphInstantiate(&exec, graph, 0);
-      cudaGraphDestroy(graph);
-      if (e3 != cudaSuccess) {
-        exec = nullptr;
-        return cuda_fail(&C, e3, "cudaGraphInstantiate");
-      }
-    }
+    cudaGraphExec_t exec = nullptr;
+    int64_t kernels = 0;
+    const int st = step_graph(C, steps, &exec, &kernels);
+    if (st != TG_OK) return st;
     TG_CUDA(&C, cudaGraphLaunch(exec, C.stream));
-    C.launches += C.graph_kernels[l][o];
+    C.launches += kernels;
     C.keys_valid = true;
     C.order_valid = true;
   }
@@ -1650,14 +1666,16 @@ int tg_autotune(tg_context* ctx, int32_t trial_steps, tg_tuning* out) {
   if (st != TG_OK) return st;
   tg_tuning best{};
   tg_get_tuning(ctx, &best);
-  best.ms_per_step = std::numeric_limits<double>::infinity();
   int timed = 0;
+  bool lists = false;  // whether the steps of the last trial ran on lists
   // Steps that trials have to repeat neither bias the next ones nor stay with
   // the context.
   const tg::ListPolicy policy = C.list_policy;
-  // Time `trial_steps` graph-replayed steps of one shape (one untimed step
-  // first captures the graph); the state goes back afterwards.
-  auto trial = [&](tg_tuning t, double* ms) -> int {
+  // Time graph-replayed steps of one shape, at least trial_steps of them and
+  // whole chains; an untimed step brings the home order that they replay in,
+  // and their graph is captured before the clock starts.  walk: on the cell
+  // walk, whose shape it is.  The state goes back afterwards.
+  auto trial = [&](tg_tuning t, bool walk, double* ms) -> int {
     *ms = std::numeric_limits<double>::infinity();
     int s = restore_snapshot(ctx, S, t.cells_per_radius);
     if (s == TG_ERR_INVALID_ARGUMENT) return TG_OK;  // grid too large: skip
@@ -1665,50 +1683,70 @@ int tg_autotune(tg_context* ctx, int32_t trial_steps, tg_tuning* out) {
     C.force_block = t.block_size;
     C.force_team = t.lanes_per_particle;
     C.list_policy = tg::ListPolicy{};
+    if (walk) C.list_policy.walk = trial_steps + 1;
     C.invalidate_graph();
     s = tg_step(ctx, 1, nullptr);
+    const int chain = C.engine->chain(C);
+    const int32_t steps = (trial_steps + chain - 1) / chain * chain;
+    if (s == TG_OK && C.use_graph && !C.profile) {
+      cudaGraphExec_t exec = nullptr;
+      int64_t kernels = 0;
+      s = step_graph(C, chain, &exec, &kernels);
+      if (s == TG_OK) TG_CUDA(&C, cudaGraphUpload(exec, C.stream));
+    }
+    lists = C.lists;
     if (s == TG_OK) s = tg_timer_start(ctx);
-    if (s == TG_OK) s = tg_step(ctx, trial_steps, nullptr);
+    if (s == TG_OK) s = tg_step(ctx, steps, nullptr);
     double total = 0.0;
     if (s == TG_OK) s = tg_timer_stop(ctx, &total);
     if (s != TG_OK) return s;
-    *ms = total / trial_steps;
+    *ms = total / steps;
     ++timed;
     return TG_OK;
   };
-  auto consider = [&](tg_tuning t) -> int {
+  // The faster of best and t, by *best_ms.
+  auto consider = [&](tg_tuning t, bool walk, double* best_ms) -> int {
     if (!valid_shape(C, t)) return TG_OK;
     double ms = 0.0;
-    const int s = trial(t, &ms);
+    const int s = trial(t, walk, &ms);
     if (s != TG_OK) return s;
-    if (ms < best.ms_per_step) {
+    if (ms < *best_ms) {
       best = t;
-      best.ms_per_step = ms;
+      *best_ms = ms;
     }
     return TG_OK;
   };
   // Coordinate search: cell size, then lanes per target, then block size,
-  // each with the others at their best so far.
+  // each with the others at their best so far.  Lanes and blocks are those of
+  // the cell walk: where steps run on lists, their trials walk.
   tg_tuning base = best;
   base.block_size = 128;
   base.lanes_per_particle = 1;
+  double ms = std::numeric_limits<double>::infinity();
   for (int k = 1; k <= 3 && st == TG_OK; ++k) {
     tg_tuning t = base;
     t.cells_per_radius = k;
-    st = consider(t);
+    st = consider(t, false, &ms);
+  }
+  const double step_ms = ms;
+  const bool walk = lists;
+  if (walk && st == TG_OK) {
+    ms = std::numeric_limits<double>::infinity();
+    st = consider(tg_tuning(best), true, &ms);
   }
   for (int lanes : {2, 4}) {
     if (st != TG_OK) break;
     tg_tuning t = best;
     t.lanes_per_particle = lanes;
-    st = consider(t);
+    st = consider(t, walk, &ms);
   }
   for (int block : {64, 256}) {
     if (st != TG_OK) break;
     tg_tuning t = best;
     t.block_size = block;
-    st = consider(t);
+    st = consider(t, walk, &ms);
   }
+  best.ms_per_step = walk ? step_ms : ms;
   // Leave the context at the best shape with the state of the call.
   const int st2 = restore_snapshot(
       ctx, S, std::isfinite(best.ms_per_step) ? best.cells_per_radius : C.k);
