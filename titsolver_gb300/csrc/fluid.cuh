@@ -2055,6 +2055,11 @@ __global__ void __launch_bounds__(128)
   if constexpr (F == TG_FP64) {
     double pa[3] = {0.0, 0.0, 0.0};
     load_pos(A.posrec, static_cast<uint32_t>(i), pa);
+    // Rows clipped to the support radius: the FP64 predicate of a candidate
+    // costs more than the clip (3D, 128,000 fluid particles 1874 -> 1686 us;
+    // the compensated form 423 / 425 us, 3D 432,000 923 / 954).
+    float oc[3] = {0.f, 0.f, 0.f};
+    cell_offset<D>(T, c, pa, oc);
     for_cells<D, false>(T, c, A.k, A.cell_start,
                         [&](uint32_t s, uint32_t en, int, int, int) {
       for (uint32_t j = s; j < en; ++j) {
@@ -2066,7 +2071,7 @@ __global__ void __launch_bounds__(128)
         hs += splitmix64(static_cast<uint64_t>(lid) + 1u);
         if (indices != nullptr) indices[out++] = static_cast<int32_t>(lid);
       }
-    });
+    }, T.cull_r2_f > 0.f ? oc : nullptr);
   } else {
     float oa[3] = {0.f, 0.f, 0.f};
     load_pos(A.posrec, static_cast<uint32_t>(i), oa);
