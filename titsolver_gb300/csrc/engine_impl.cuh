@@ -20,8 +20,7 @@ inline unsigned grid_for(int64_t n, int block) {
 
 // Compile-time physics preset of the compensated force kernel for params.
 inline int physics_preset(const tg_params& P) {
-  // The presets' pair sums take the Tait law with xi = 7 for granted.
-  if (!P.kahan || P.xi != 7.0 || P.eos != TG_EOS_TAIT) return kPhysGeneric;
+  if (!P.kahan) return kPhysGeneric;
   if (P.viscosity == TG_VISC_MONAGHAN && P.diffusion == TG_DIFF_MOLTENI) {
     return kPhysTextbook;
   }
@@ -29,6 +28,14 @@ inline int physics_preset(const tg_params& P) {
     return kPhysReference;
   }
   return kPhysGeneric;
+}
+
+// That of the pair sums on lists.  In 3D, where a record holds no sound speed,
+// the presets take the Tait law with xi = 7 for granted.
+template<int D>
+int list_preset(const tg_params& P) {
+  const bool law = D == 2 || (P.xi == 7.0 && P.eos == TG_EOS_TAIT);
+  return law ? physics_preset(P) : kPhysGeneric;
 }
 
 // Longest list of a particle.
@@ -487,7 +494,7 @@ class Engine final : public EngineBase {
       }
       tok = C.group_begin(kGroupForces);
       if constexpr (F == TG_FP32C) {
-        const int phys = physics_preset(C.P);
+        const int phys = list_preset<D>(C.P);
         if (phys == kPhysTextbook) {
           launch_list_forces<kPhysTextbook>(C, A, team);
         } else if (phys == kPhysReference) {
