@@ -455,29 +455,32 @@ int upload_particles(tg_context* ctx, int32_t n_tanks, const tg_tank* tanks,
     }
   }
 
-  // Per-tank grids.
-  std::vector<tg::TankDev> td(static_cast<size_t>(n_tanks));
-  std::vector<uint32_t> id_base(static_cast<size_t>(n_tanks));
-  std::vector<uint32_t> wall_from(static_cast<size_t>(n_tanks));
-  uint64_t total_cells = 0;
+  // Bounding boxes, and whether steps will run on neighbour lists as far as
+  // can be told now (a wrong guess costs only speed).  Their cells are a
+  // twentieth wider than R / k: the lists' radius (pairlist.cuh) then stays
+  // within k cells while particles move 2.5% of R per step, and the outer ring
+  // of rows need not be looked at (sort + build 1.23 -> 1.19 ms at 2M fluid
+  // particles in 3D, .385 -> .354 at 1.28M in 2D; 3% and 7% gained less).
+  // Steps that walk cells take cells of R / k (ms per step on the wider cells
+  // and on these: symplectic Euler, 3D 432k fluid compensated 1.230 / 1.174,
+  // 2D 500k .603 / .561, FP64 3D 128k 7.87 / 7.18; Verlet there 1.854 / 1.772,
+  // .897 / .837, 12.05 / 10.93; SSPRK3 without room for lists, 3D 128k FP64
+  // 12.58 / 11.07, 432k compensated 1.947 / 1.831), except SSPRK in 2D (500k
+  // compensated .829 / .982 near a lattice, .936 / .986 in disorder; FP64
+  // 13.7 / 15.3 and 15.5 / 15.2).
+  std::vector<std::array<double, 6>> box(static_cast<size_t>(n_tanks));  // lows, highs
+  size_t avail = 0, device_total = 0;
+  TG_CUDA(&C, cudaMemGetInfo(&avail, &device_total));
+  double entries = 0.0;
+  const bool ssprk = C.P.integrator == TG_SSPRK3 || C.P.integrator == TG_SSPRK2;
+  bool wide = ssprk && nf > 0;
   int64_t base = 0;
   for (int32_t t = 0; t < n_tanks; ++t) {
     const tg_tank& T = tanks[t];
     const int64_t nt = T.n_fluid + T.n_wall;
-    tg::TankDev& D = td[t];
-    std::memset(&D, 0, sizeof(D));
     const double R = tg::kernel_unit_radius(C.P.kernel) * T.h;
-    // A twentieth wider than R / k: the lists' radius (pairlist.cuh) then
-    // stays within k cells while particles move 2.5% of R per step, and the
-    // outer ring of rows need not be looked at (sort + build 1.23 -> 1.19 ms
-    // at 2M fluid particles in 3D, .385 -> .354 at 1.28M in 2D; 3% and 7%
-    // gained less).  The integrators without lists walk cells of R / k
-    // (ms per step on the wider cells and on these: symplectic Euler, 3D 432k
-    // fluid compensated 1.230 / 1.174, 2D 500k .603 / .561, FP64 3D 128k
-    // 7.87 / 7.18; Verlet there 1.854 / 1.772, .897 / .837, 12.05 / 10.93).
-    const bool ssprk = C.P.integrator == TG_SSPRK3 || C.P.integrator == TG_SSPRK2;
-    const double cs = R / C.k * (ssprk ? 1.0 + 1.0 / 20.0 : 1.0 + 1.0 / 65536.0);
-    double lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
+    double *lo = box[t].data(), *hi = lo + 3;
+    double extent = 0.0;
     if (nt > 0) {
       for (int k = 0; k < dim; ++k) lo[k] = hi[k] = r[base * dim + k];
       for (int64_t i = base; i < base + nt; ++i) {
@@ -487,103 +490,134 @@ int upload_particles(tg_context* ctx, int32_t n_tanks, const tg_tank* tanks,
         }
       }
     }
-    // Headroom above the tank for splashes (particles beyond the grid are
-    // clamped into its border cells, which stays exact but slows them).
-    // Margins of R + 2 cells keep every particle's block of cells within k
-    // of its own off the border cells.
-    const double headroom = 0.25 * (hi[1] - lo[1]);
-    uint64_t cells = 1;
-    for (int k = 0; k < 3; ++k) {
-      if (k < dim) {
-        D.lo[k] = lo[k] - (R + 2.0 * cs);
-        double top = hi[k] + (R + 2.0 * cs) + (k == 1 ? headroom : 0.0);
-        const double ncf = std::max(1.0, std::ceil((top - D.lo[k]) / cs));
-        if (ncf > 2.0e9) {
-          return fail(&C, TG_ERR_INVALID_ARGUMENT, "tank grid too large");
-        }
-        D.nc[k] = static_cast<int32_t>(ncf);
-      } else {
-        D.lo[k] = 0.0;
-        D.nc[k] = 1;
-      }
-      cells *= static_cast<uint64_t>(D.nc[k]);
-    }
-    D.cs = cs;
-    D.inv_cs = 1.0 / cs;
-    D.cell_off = static_cast<uint32_t>(total_cells);
-    total_cells += cells;
-    if (total_cells >= (uint64_t{1} << 30)) {
-      return fail(&C, TG_ERR_INVALID_ARGUMENT,
-                  "more than 2^30 grid cells; lower cells_per_radius");
-    }
-    D.h = T.h;
-    D.hinv = 1.0 / T.h;
-    D.radius2 = R * R;
-    const float hf = static_cast<float>(T.h);
-    const float Rf = static_cast<float>(tg::kernel_unit_radius(C.P.kernel)) * hf;
-    D.radius2_f = Rf * Rf;
-    D.band_lo_f = static_cast<float>(R * R * (1.0 - 1.0 / 16384.0));
-    D.band_hi_f = static_cast<float>(R * R * (1.0 + 1.0 / 16384.0));
-    D.cs_f = static_cast<float>(cs);
-    D.inv_cs_f = static_cast<float>(1.0 / cs);
-    double hinv_d = 1.0;
-    for (int k = 0; k < dim; ++k) hinv_d *= D.hinv;
-    D.w = kernel_weight(C.P.kernel, dim) * hinv_d;
-    D.wg = D.w * D.hinv;
-    D.m = T.m;
-    D.rho0 = T.rho0;
-    D.cs0 = T.cs0;
-    D.B = T.rho0 * T.cs0 * T.cs0 / C.P.xi;
-    D.diff_k = 2.0 * C.P.delta * T.h * T.cs0;
-    D.visc_eps2 = 0.01 * T.h * T.h;
-    D.n_fluid = static_cast<uint32_t>(T.n_fluid);
-    D.h_f = static_cast<float>(D.h);
-    D.hinv_f = static_cast<float>(D.hinv);
-    D.w_f = static_cast<float>(D.w);
-    D.wg_f = static_cast<float>(D.wg);
-    D.m_f = static_cast<float>(D.m);
-    D.rho0_f = static_cast<float>(D.rho0);
-    D.cs0_f = static_cast<float>(D.cs0);
-    D.B_f = static_cast<float>(D.B);
-    D.diff_k_f = static_cast<float>(D.diff_k);
-    D.visc_eps2_f = static_cast<float>(D.visc_eps2);
-    D.c02_f = static_cast<float>(D.cs0 * D.cs0);
-    {
-      const double unit = cs / 268435456.0;  // 2^-28 cells
-      const bool wendland = C.P.kernel >= TG_KERNEL_WENDLAND_C2;
-      // f'(q)/q of the Wendland kernels without the polynomial of list_g.
-      const double lead = C.P.kernel == TG_KERNEL_WENDLAND_C2   ? -5.0
-                          : C.P.kernel == TG_KERNEL_WENDLAND_C4 ? -14.0 / 3.0
-                                                                : -2.75;
-      D.list_inv_unit = 1.0 / unit;
-      D.list_s = wendland ? T.m * D.wg * D.hinv * lead : T.m * D.wg;
-      D.list_s_f = static_cast<float>(wendland ? D.list_s * unit : D.list_s);
-      D.list_unit_f = static_cast<float>(unit);
-      D.list_hq_f = static_cast<float>(unit * D.hinv);
-      D.list_ah_f = static_cast<float>(C.P.alpha * T.h / unit);
-      D.list_eps2_f = static_cast<float>(D.visc_eps2 / (unit * unit));
-      D.list_dk_f = static_cast<float>(D.diff_k / unit);
-      D.list_mu2_f = static_cast<float>(2.0 * C.P.mu / unit);
-      D.list_lo_f = static_cast<float>(R * R * (1.0 - 1.0 / 16384.0) / (unit * unit));
-      D.list_hi_f = static_cast<float>(R * R * (1.0 + 1.0 / 16384.0) / (unit * unit));
-      D.R_f = static_cast<float>(R);
-      D.inv_rho0_f = static_cast<float>(1.0 / T.rho0);
-    }
-    {
-      const double rc = R * (1.0 + 1.0 / 4096.0);
-      D.cull_r2_f = static_cast<float>(rc * rc);
-      double extent = 0.0;
-      for (int k = 0; k < dim; ++k) extent = std::max(extent, D.nc[k] * cs);
-      const double rs = rc + extent / 524288.0;
-      D.wall_skip_r2_f = static_cast<float>(rs * rs);
-      // Rounding of the tank-local FP32 coordinates, of the row clips and
-      // of the squared distance: 8 ulps of the extent and R / 2048.
-      D.list_slack_f = static_cast<float>(extent / 2097152.0 + R / 2048.0);
-    }
-    id_base[t] = static_cast<uint32_t>(base);
-    wall_from[t] = static_cast<uint32_t>(base + T.n_fluid);
+    for (int k = 0; k < dim; ++k) extent = std::max(extent, 1.25 * (hi[k] - lo[k]) + 6.0 * R);
+    entries = std::max(entries, tg::list_entries(dim, R, T.rho0, T.m));
+    wide = wide && tg::list_resolved(R, tg::list_slack(extent, R));
     base += nt;
   }
+  const double cap = tg::list_capacity(entries, 1.0);
+  wide = wide && cap <= tg::kListMaxCap &&
+         (4.0 * cap + 100.0) * static_cast<double>(n) <=
+             0.35 * (static_cast<double>(device_total) - 700.0 * static_cast<double>(n));
+  wide = wide || (ssprk && dim == 2);
+
+  // Per-tank grids.
+  std::vector<tg::TankDev> td(static_cast<size_t>(n_tanks));
+  std::vector<uint32_t> id_base(static_cast<size_t>(n_tanks));
+  std::vector<uint32_t> wall_from(static_cast<size_t>(n_tanks));
+  uint64_t total_cells = 0;
+  const auto make_grids = [&](bool wide_cells) -> int {
+    total_cells = 0;
+    base = 0;
+    for (int32_t t = 0; t < n_tanks; ++t) {
+      const tg_tank& T = tanks[t];
+      const int64_t nt = T.n_fluid + T.n_wall;
+      tg::TankDev& D = td[t];
+      std::memset(&D, 0, sizeof(D));
+      const double R = tg::kernel_unit_radius(C.P.kernel) * T.h;
+      const double cs = R / C.k * (wide_cells ? 1.0 + 1.0 / 20.0 : 1.0 + 1.0 / 65536.0);
+      const double *lo = box[t].data(), *hi = lo + 3;
+      // Headroom above the tank for splashes (particles beyond the grid are
+      // clamped into its border cells, which stays exact but slows them).
+      // Margins of R + 2 cells keep every particle's block of cells within k
+      // of its own off the border cells.
+      const double headroom = 0.25 * (hi[1] - lo[1]);
+      uint64_t cells = 1;
+      for (int k = 0; k < 3; ++k) {
+        if (k < dim) {
+          D.lo[k] = lo[k] - (R + 2.0 * cs);
+          double top = hi[k] + (R + 2.0 * cs) + (k == 1 ? headroom : 0.0);
+          const double ncf = std::max(1.0, std::ceil((top - D.lo[k]) / cs));
+          if (ncf > 2.0e9) {
+            return fail(&C, TG_ERR_INVALID_ARGUMENT, "tank grid too large");
+          }
+          D.nc[k] = static_cast<int32_t>(ncf);
+        } else {
+          D.lo[k] = 0.0;
+          D.nc[k] = 1;
+        }
+        cells *= static_cast<uint64_t>(D.nc[k]);
+      }
+      D.cs = cs;
+      D.inv_cs = 1.0 / cs;
+      D.cell_off = static_cast<uint32_t>(total_cells);
+      total_cells += cells;
+      if (total_cells >= (uint64_t{1} << 30)) {
+        return fail(&C, TG_ERR_INVALID_ARGUMENT,
+                    "more than 2^30 grid cells; lower cells_per_radius");
+      }
+      D.h = T.h;
+      D.hinv = 1.0 / T.h;
+      D.radius2 = R * R;
+      const float hf = static_cast<float>(T.h);
+      const float Rf = static_cast<float>(tg::kernel_unit_radius(C.P.kernel)) * hf;
+      D.radius2_f = Rf * Rf;
+      D.band_lo_f = static_cast<float>(R * R * (1.0 - 1.0 / 16384.0));
+      D.band_hi_f = static_cast<float>(R * R * (1.0 + 1.0 / 16384.0));
+      D.cs_f = static_cast<float>(cs);
+      D.inv_cs_f = static_cast<float>(1.0 / cs);
+      double hinv_d = 1.0;
+      for (int k = 0; k < dim; ++k) hinv_d *= D.hinv;
+      D.w = kernel_weight(C.P.kernel, dim) * hinv_d;
+      D.wg = D.w * D.hinv;
+      D.m = T.m;
+      D.rho0 = T.rho0;
+      D.cs0 = T.cs0;
+      D.B = T.rho0 * T.cs0 * T.cs0 / C.P.xi;
+      D.diff_k = 2.0 * C.P.delta * T.h * T.cs0;
+      D.visc_eps2 = 0.01 * T.h * T.h;
+      D.n_fluid = static_cast<uint32_t>(T.n_fluid);
+      D.h_f = static_cast<float>(D.h);
+      D.hinv_f = static_cast<float>(D.hinv);
+      D.w_f = static_cast<float>(D.w);
+      D.wg_f = static_cast<float>(D.wg);
+      D.m_f = static_cast<float>(D.m);
+      D.rho0_f = static_cast<float>(D.rho0);
+      D.cs0_f = static_cast<float>(D.cs0);
+      D.B_f = static_cast<float>(D.B);
+      D.diff_k_f = static_cast<float>(D.diff_k);
+      D.visc_eps2_f = static_cast<float>(D.visc_eps2);
+      D.c02_f = static_cast<float>(D.cs0 * D.cs0);
+      {
+        const double unit = cs / 268435456.0;  // 2^-28 cells
+        const bool wendland = C.P.kernel >= TG_KERNEL_WENDLAND_C2;
+        // f'(q)/q of the Wendland kernels without the polynomial of list_g.
+        const double lead = C.P.kernel == TG_KERNEL_WENDLAND_C2   ? -5.0
+                            : C.P.kernel == TG_KERNEL_WENDLAND_C4 ? -14.0 / 3.0
+                                                                  : -2.75;
+        D.list_inv_unit = 1.0 / unit;
+        D.list_s = wendland ? T.m * D.wg * D.hinv * lead : T.m * D.wg;
+        D.list_s_f = static_cast<float>(wendland ? D.list_s * unit : D.list_s);
+        D.list_unit_f = static_cast<float>(unit);
+        D.list_hq_f = static_cast<float>(unit * D.hinv);
+        D.list_ah_f = static_cast<float>(C.P.alpha * T.h / unit);
+        D.list_eps2_f = static_cast<float>(D.visc_eps2 / (unit * unit));
+        D.list_dk_f = static_cast<float>(D.diff_k / unit);
+        D.list_mu2_f = static_cast<float>(2.0 * C.P.mu / unit);
+        D.list_lo_f = static_cast<float>(R * R * (1.0 - 1.0 / 16384.0) / (unit * unit));
+        D.list_hi_f = static_cast<float>(R * R * (1.0 + 1.0 / 16384.0) / (unit * unit));
+        D.R_f = static_cast<float>(R);
+        D.inv_rho0_f = static_cast<float>(1.0 / T.rho0);
+      }
+      {
+        const double rc = R * (1.0 + 1.0 / 4096.0);
+        D.cull_r2_f = static_cast<float>(rc * rc);
+        double extent = 0.0;
+        for (int k = 0; k < dim; ++k) extent = std::max(extent, D.nc[k] * cs);
+        const double rs = rc + extent / 524288.0;
+        D.wall_skip_r2_f = static_cast<float>(rs * rs);
+        D.list_slack_f = static_cast<float>(tg::list_slack(extent, R));
+      }
+      id_base[t] = static_cast<uint32_t>(base);
+      wall_from[t] = static_cast<uint32_t>(base + T.n_fluid);
+      base += nt;
+    }
+    return TG_OK;
+  };
+  int st = make_grids(wide);
+  // What only the wider cells keep below the limits takes them.
+  if (st != TG_OK && !wide && ssprk) st = make_grids(true);
+  if (st != TG_OK) return st;
 
   // (Re)allocate.
   cudaStreamSynchronize(C.stream);

@@ -2,6 +2,7 @@
 // the per-(dimension, form, kernel) templates implement.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <memory>
 #include <string>
@@ -23,6 +24,23 @@ struct Context;
 // 2.44 / 3.02 / 3.03, 24 3D tanks 1.68 / 1.39 / 1.84 / 1.98, 2D 1.28M 0.969 /
 // 0.854 / 0.849 / 0.815.
 constexpr int kListChain = 2;
+
+// Longest list of a particle, and the room for one: the entries of a ball of
+// the list's radius at the reference density (1.1 R; the largest over the
+// tanks), with room for disorder and compression.
+constexpr double kListMaxCap = 1024.0;
+inline double list_entries(int dim, double R, double rho0, double m) {
+  const double a = 1.1 * R;
+  return (dim == 2 ? 3.14159265358979 * a * a : 4.18879020478639 * a * a * a) * rho0 / m;
+}
+inline double list_capacity(double entries, double room) {
+  return std::ceil((1.3 * entries + 12.0) * room / 4.0) * 4.0;
+}
+// Whether tank-local FP32 coordinates resolve a radius (slack: their rounding).
+inline bool list_resolved(double R, double slack) { return slack <= 0.02 * R; }
+// Rounding of the tank-local FP32 coordinates, of the row clips and of the
+// squared distance: 8 ulps of the extent and R / 2048.
+inline double list_slack(double extent, double R) { return extent / 2097152.0 + R / 2048.0; }
 
 // Force passes per step of an integrator.
 inline int force_passes(int integrator) {

@@ -38,9 +38,6 @@ int list_preset(const tg_params& P) {
   return law ? physics_preset(P) : kPhysGeneric;
 }
 
-// Longest list of a particle.
-constexpr double kListMaxCap = 1024.0;
-
 // Kernels with multi-lane force variants: the two the shipped parameter
 // sets use (Wendland C2 and C4); the others run one lane per target.
 constexpr bool team_kernel(int K) {
@@ -353,19 +350,12 @@ class Engine final : public EngineBase {
 
   // Takes the buffers of the list steps; false where they do not fit.
   bool take_lists(Context& C) {
-    // Entries per particle: those of a ball of the list's radius at the
-    // reference density, with room for disorder and compression; the
-    // largest over the tanks.
     double most = 0.0;
-    for (size_t t = 0; t < C.tanks.size(); ++t) {
-      const TankDev& T = C.tankdev[t];
-      const double R = 1.1 * T.R_f;
-      const double ball = D == 2 ? 3.14159265358979 * R * R : 4.18879020478639 * R * R * R;
-      most = std::max(most, ball * T.rho0 / T.m);
-      // Tank-local FP32 coordinates must resolve the radius.
-      if (T.list_slack_f > 0.02f * T.R_f) return false;
+    for (const TankDev& T : C.tankdev) {
+      most = std::max(most, list_entries(D, T.R_f, T.rho0, T.m));
+      if (!list_resolved(T.R_f, T.list_slack_f)) return false;
     }
-    const double cap = std::ceil((1.3 * most + 12.0) * C.list_policy.room / 4.0) * 4.0;
+    const double cap = list_capacity(most, C.list_policy.room);
     if (!(cap <= kListMaxCap)) return false;
     C.list_cap = static_cast<int>(cap);
     const size_t n = static_cast<size_t>(C.n), slots = 32 * ((n + 31) / 32);
