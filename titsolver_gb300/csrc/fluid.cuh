@@ -2154,7 +2154,7 @@ __global__ void __launch_bounds__(128) k_gamma_init(StageArgs<D, F> A) {
 
 template<int D, int K, int F, class FT>
 __global__ void __launch_bounds__(128) k_gamma_faces(StageArgs<D, F> A) {
-  __shared__ uint32_t flist_all[kFaceBlock / face_group<D>()][kFaceListCap<D>];
+  __shared__ uint32_t flist_all[kFaceBlock / face_group<D>()][kFaceListCap];
   const FaceArgs& fc = A.fc;
   constexpr int G = face_group<D>();
   const int lane = face_lane<D>();
@@ -2179,9 +2179,9 @@ __global__ void __launch_bounds__(128) k_gamma_faces(StageArgs<D, F> A) {
     // sweep at xs keeps the adjacency of x); the skip masks come from the
     // same list.  Past the list's capacity both sweeps test the cell list
     // again, as for_adjacent_faces does.
-    const int nf = collect_adjacent_faces<D>(fc, gcell, x, radius, lane, flist, kFaceListCap<D>);
+    const int nf = collect_adjacent_faces<D>(fc, gcell, x, radius, lane, flist, kFaceListCap);
     auto sweep = [&](auto&& fn) {
-      if (nf <= kFaceListCap<D>) {
+      if (nf <= kFaceListCap) {
         for (int base = 0; base < nf; base += G) {
           const bool active = base + lane < nf;
           const uint32_t fi = flist[active ? base + lane : base];
