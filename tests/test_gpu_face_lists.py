@@ -37,3 +37,21 @@ def test_segments_around_the_list(gpu_lib, finer):
         g = gpu_state(ctx)
     for key in ("r", "v", "rho"):
         assert rel_l2(g[key][f], getattr(o, key)[f]) <= 1e-11, key
+
+
+@pytest.mark.parametrize("precision", (_abi.TG_FP64, _abi.TG_FP32C))
+def test_dropped_faces_leave_the_steps(gpu_lib, precision):
+    # Steps replay graphs: those with faces go with the faces.
+    scn = scenarios.dam_break_2d_faces(nx_per_H=20)
+    P = physics.reference_params(2, precision=precision)
+    out = []
+    for faces in (True, False):
+        with gpu_context(scn if faces else dict(scn, faces=None), P) as ctx:
+            if faces:
+                ctx.step(5)
+                ctx.set_faces(0, np.empty((0, 2)), np.empty((0, 2)))
+            ctx.update(scn["r"], scn["v"], scn["rho"])
+            ctx.step(5)
+            out.append(gpu_state(ctx))
+    for key in ("r", "v", "rho"):
+        np.testing.assert_array_equal(out[0][key], out[1][key])

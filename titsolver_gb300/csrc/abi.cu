@@ -1227,6 +1227,8 @@ double winding_number3(const std::vector<double>& tris, size_t first, size_t cou
 int build_faces(tg_context* ctx) {
   Context& C = ctx->c;
   C.faces = tg::FaceArgs{};
+  C.invalidate_graph();  // also when no faces are left
+  C.walls_fresh = false;
   bool any = false;
   for (const auto& t : C.face_host) any = any || !t.face_verts.empty();
   if (!any) return TG_OK;
@@ -1522,8 +1524,6 @@ int build_faces(tg_context* ctx) {
   fa.on = 1;
   TG_CUDA(&C, cudaStreamSynchronize(C.stream));
   C.faces = fa;
-  C.invalidate_graph();
-  C.walls_fresh = false;
   return TG_OK;
 }
 
