@@ -479,7 +479,7 @@ int upload_particles(tg_context* ctx, int32_t n_tanks, const tg_tank* tanks,
     const tg_tank& T = tanks[t];
     const int64_t nt = T.n_fluid + T.n_wall;
     const double R = tg::kernel_unit_radius(C.P.kernel) * T.h;
-    double *lo = box[t].data(), *hi = lo + 3;
+    double lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
     double extent = 0.0;
     if (nt > 0) {
       for (int k = 0; k < dim; ++k) lo[k] = hi[k] = r[base * dim + k];
@@ -490,6 +490,7 @@ int upload_particles(tg_context* ctx, int32_t n_tanks, const tg_tank* tanks,
         }
       }
     }
+    box[t] = {lo[0], lo[1], lo[2], hi[0], hi[1], hi[2]};
     for (int k = 0; k < dim; ++k) extent = std::max(extent, 1.25 * (hi[k] - lo[k]) + 6.0 * R);
     entries = std::max(entries, tg::list_entries(dim, R, T.rho0, T.m));
     wide = wide && tg::list_resolved(R, tg::list_slack(extent, R));
