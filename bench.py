@@ -268,13 +268,23 @@ def forces_compute(dim: int, n_fluid: int, pairs: int, avg_ms: float,
 
 
 def forces_ceiling(dim: int, form: str) -> dict | None:
-    """The unit that bounds k_list_forces in its ncu capture (issue slots for the
-    compensated form, the FP64 pipe for the plain one) and how busy it was:
+    """The instruction side of k_list_forces in its ncu capture (issue slots for
+    the compensated form, the FP64 pipe for the plain one) and how busy it was:
     a recorded capture, beside the live HBM fraction."""
     d = _forces_profile(dim, form)
     if d is None or "working_ceiling" not in d:
         return None
     return {**d["working_ceiling"], "source": d["source"]}
+
+
+def forces_bound(dim: int, form: str) -> dict | None:
+    """The unit that bounds k_list_forces in the same capture: the L1's
+    throughput for the compensated form's record gathers (with the issue slots
+    beside it), the FP64 pipe for the plain one."""
+    c, d = forces_ceiling(dim, form), _forces_profile(dim, form)
+    if c is None or "bound" not in d:
+        return c
+    return {**d["bound"], "source": d["source"], "instruction_side": c}
 
 
 def sample_scenario(dim: int, nx: int, cfg: str | None = None):
@@ -623,7 +633,7 @@ def run_gpu(args, ranks) -> dict | None:
                 "alg_bytes_per_launch": alg, "avg_launch_ms": forces_avg_ms,
                 "compute": forces_compute(dim, nf, pairs, forces_avg_ms, clk,
                                           tuning32.get("cells_per_radius")),
-                "ncu_working_ceiling": forces_ceiling(dim, "fp32c")}
+                "ncu_working_ceiling": forces_bound(dim, "fp32c")}
 
     extras = {}
     for name in [x for x in args.extra.split(",") if x and x != args.config]:

@@ -145,11 +145,12 @@ typedef struct tg_params {
   int32_t cells_per_radius; /* grid cells per support radius, 1..3 */
   int32_t kahan;            /* FP32C: 1 = compensated sums, 0 = plain */
   int32_t device;           /* CUDA device ordinal; -1 = the current one */
-  int32_t staging;          /* 2D FP32C, in the force passes that walk
-                               cells (see tg_step): copy each block's
-                               neighbour window into shared memory with
-                               bulk copies (1) or read it through L1 (0,
-                               default; measured faster on GB300) */
+  int32_t staging;          /* 2D FP32C force passes that walk cells: copy
+                               each block's neighbour window into shared
+                               memory with bulk copies (1) or read it
+                               through L1 (0, default; measured faster on
+                               GB300).  No effect on SSPRK steps that run on
+                               neighbour lists (see tg_step). */
   int32_t eos;              /* TG_EOS_TAIT (default) | TG_EOS_LINEAR_TAIT */
   int32_t face_fp32;        /* TG_FP32C with face walls: the closed-form face
                                integrals in FP32 (1) or FP64 (0, default).
@@ -227,10 +228,13 @@ int tg_prepare(tg_context* ctx);
 /* Advance every tank by n_steps integrator steps (each with its own dt).
  * dt_out (n_tanks doubles, may be NULL) receives the last step's dt.
  * SSPRK3 and SSPRK2 steps run on neighbour lists that hold for one step, or
- * for two steps of one call.  Steps whose particles leave the lists' reach
- * or overflow them are repeated with a sort and a cell walk per stage, which
- * the other integrators, and particle sets whose lists would take more than
- * a third of the free device memory, use throughout. */
+ * for two steps of one call.  Where particles leave the lists' reach or
+ * overflow them, the steps that share those lists are repeated with a sort
+ * and a cell walk per stage, and the call goes on with lists.  The other
+ * integrators walk cells throughout, and so do particle sets whose lists
+ * would take more than a third of the free device memory (decided at the
+ * first step after an upload) or whose extent is beyond 40,000 support
+ * radii. */
 int tg_step(tg_context* ctx, int32_t n_steps, double* dt_out);
 
 /* Per-tank accumulated time (n_tanks doubles). */
@@ -362,7 +366,7 @@ int tg_tank_faces(tg_context* ctx, int32_t tank, int32_t n_faces,
  * passes that walk cells, the threads per block and the lanes per fluid
  * particle (1, 2 or 4: the lanes split the particle's neighbour cells, so a
  * warp advances 32, 16 or 8 particles; 2 and 4 exist for the Wendland C2 and
- * C4 kernels).  Force passes on neighbour lists choose their own. */
+ * C4 kernels).  Passes on neighbour lists choose theirs by the run's size. */
 typedef struct tg_tuning {
   int32_t cells_per_radius;   /* 1..3 */
   int32_t block_size;         /* 64, 128 or 256 */

@@ -20,9 +20,12 @@ struct Context;
 
 // Steps of a chain (pairlist.cuh).  Longer chains spread the sort, gather and
 // list build over more steps and make every pair pass walk wider lists.
-// Measured in ms per step at 1 / 2 / 3 / 4 steps: 3D 2M fluid particles 2.85 /
-// 2.44 / 3.02 / 3.03, 24 3D tanks 1.68 / 1.39 / 1.84 / 1.98, 2D 1.28M 0.969 /
-// 0.854 / 0.849 / 0.815.
+// Measured in ms per step at 1 / 2 / 3 / 4 steps: 2D 1.28M fluid particles
+// 0.969 / 0.854 / 0.849 / 0.815; 3D 2M 2.85 / 2.44 / 3.02 / 3.03, 24 3D tanks
+// 1.68 / 1.39 / 1.84 / 1.98.  The 3D times at 3 and 4 steps are not those of
+// the chain alone: their lists outgrew the room (that of 1.1 R, whatever the
+// chain) and steps were repeated.  2 in both dimensions; 4 in 2D, 5% faster,
+// has not been taken up.
 constexpr int kListChain = 2;
 
 // Longest list of a particle, and the room for one: the entries of a ball of

@@ -13,12 +13,14 @@
 //               update, SSPRK linear combination, and the cell key (and
 //               FP32 cell offset) of the new position for the next sort
 //               (fluid_equations.hpp:232-305, time_integrator.hpp:203-223)
-// The last pass over the particles writes their keys by fixed-point
-// arithmetic (cell_and_offset); k_keys computes them from FP64 positions only
-// after an upload or update (FP64 issue is scarce on GB300).
+// The last pass over the particles writes the keys of their new positions
+// (commit_fluid: cell_of in the plain form, a step of whole cells from the old
+// one in the compensated form); k_keys computes them from the positions after
+// an upload or update, by fixed-point arithmetic (cell_and_offset).
 // SSPRK steps run these stages only where the neighbour lists of
 // pairlist.cuh do not serve: steps that the lists' bounds stop, and sets
-// whose lists would take too much memory.  The other integrators, and the
+// whose lists would take too much memory or whose radius tank-local FP32
+// coordinates do not resolve.  The other integrators, and the
 // prepare passes outside a step, always run them.
 #pragma once
 

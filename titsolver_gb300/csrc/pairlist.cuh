@@ -17,7 +17,8 @@
 // margin for the accelerations, and every stage checks it: a particle beyond
 // delta, or a list past its capacity, raises *stop.  The last stage and all
 // later kernels then leave the home state as the step found it, and the host
-// repeats the step with a sort per stage (tg_step).  Nothing is approximated:
+// repeats the step, or its chain, with a sort per stage and goes on with lists
+// (tg_step, listpolicy.cuh).  Nothing is approximated:
 // every entry's |r_ab| is taken anew in every stage, and an entry beyond R
 // adds nothing: by the predicate |r_ab| <= R, or, in the compensated form
 // with a Wendland kernel, by the kernel itself, whose clamped factor
@@ -30,10 +31,11 @@
 // is written by the chain's last step, so a stop repeats the whole chain.
 //
 // Positions of the compensated form are 32-bit fixed point, in units of
-// 2^-28 cells modulo 2^32: a difference is exact while it is below 8 cells
-// (listed pairs are within R + 2 delta <= 1.5 R <= 4.5 cells), whatever the
-// cells of the two particles are, so no cell offsets enter the pair loop and
-// r_ab keeps the relative precision of FP32.  The unit stays in the pair
+// 2^-28 cells modulo 2^32: a difference is exact while it is below 8 cells,
+// whatever the cells of the two particles are, so no cell offsets enter the
+// pair loop and r_ab keeps the relative precision of FP32.  (A listed pair is
+// within R + 2 delta when the lists are built and each of the two then moves
+// delta <= R / 4 at most: R + 4 delta <= 2 R <= 6 cells at 3 cells per radius.)  The unit stays in the pair
 // loop; the constants absorb it.
 #pragma once
 
@@ -743,8 +745,9 @@ struct ListPairF32 {
 // FP64 form, one target.  GB300's FP64 pipe bounds this form, so the pair
 // costs as few FP64 operations as the sums allow: one reciprocal square root
 // and one quotient, each from the hardware seed (relative error below 2^-19)
-// by one third-order iteration in the residual e (truncation e^3, below
-// 2^-56), and comparisons on the high words.
+// by the third-order iteration of rcp_f64 and sqrt_f64 in the residual e
+// (truncation 5 e^3 / 16 < 2^-55 and e^3 < 2^-57), and comparisons on the high
+// words.
 template<int D, int F, int K>
 struct ListPairF64 {
   Dat64 a;
@@ -848,7 +851,6 @@ template<int D, int F, int K, int Team>
 __global__ void __launch_bounds__(128) k_list_walls(ListArgs<D, F> A) {
   if (*A.stop != 0u) return;
   const StageArgs<D, F>& S = A.S;
-  using R = typename StageArgs<D, F>::R;
   const bool all = S.fbox == nullptr;
   const uint32_t* list = all ? S.wall_list : S.wall_active;
   const int64_t count = all ? S.wall_count[0] : S.wall_count[1];
@@ -934,7 +936,6 @@ __global__ void __launch_bounds__(128) k_list_walls(ListArgs<D, F> A) {
         A.dat_in[ew] = rec;
       }
     }
-    (void)sizeof(R);
   }
 }
 
