@@ -1316,7 +1316,9 @@ int build_faces(tg_context* ctx) {
     const size_t ntri = F.poly.size() / 9;
     cont_tri.insert(cont_tri.end(), F.poly.begin(), F.poly.end());
     tank_edges[t] = static_cast<uint32_t>(ntri);
-    const double hair = 1e-9 * T.cs;
+    // Wider than the fixed point's rounding (2^-29 cells), by which k_keys may
+    // put a particle into the next cell.
+    const double hair = 4e-9 * T.cs;
     for (size_t i = 0; i < ntri; ++i) {
       const double* tri = F.poly.data() + 9 * i;
       int c0[3], c1[3];
